@@ -28,7 +28,7 @@
 // the online form in fp32 in the log2 domain; column statistics are reduced with warp shuffles.
 //
 // Generic path (any dtype / head_dim <= 256 / block size): one CTA per (sequence, query head),
-// fp32 FMA arithmetic.  It is the path the fp32 engine configuration uses.
+// fp32 FMA arithmetic.  fp32 at head sizes 32 / 64 / 128 runs decode_f32.cu instead.
 //
 // SIGM variants of both: the weights are sigmoid(scale q.k + bias[head]) and are not normalised, only the keys of the last
 // token's chunk of positions are listed and read, pieces of a cut sequence just add up, and a row leaves through its gate.
@@ -822,6 +822,11 @@ extern "C" size_t b200_paged_decode_gqa_workspace_bytes(int32_t batch, int32_t n
 }
 
 namespace b200 {
+// fp32 at head sizes 32 / 64 / 128 (decode_f32.cu)
+int decode_f32_launch(const void* q, const void* kc, const void* vc, void* out, const int32_t* bt, int64_t bt_stride,
+                      const int64_t* lens, int batch, int Hq, int Hkv, int D, int Dv, int bs, int64_t num_blocks,
+                      float scale_log2, const float* sink, int32_t* status, cudaStream_t s);
+
 namespace {
 // what the sigmoid form has in addition
 struct SigmoidForm {
@@ -918,6 +923,11 @@ static int paged_decode(const void* q, const void* k_cache, const void* v_cache,
   }
 
   if (head_dim > kSimpleMaxPerLane * 32 || head_dim_v > kSimpleMaxPerLane * 32) return B200_ERR_UNSUPPORTED;
+  if (!SIGM && dtype == B200_DTYPE_F32) {
+    const int rc = decode_f32_launch(q, k_cache, v_cache, out, block_tables, bt_stride, context_lens, batch, num_q_heads,
+                                     num_kv_heads, head_dim, head_dim_v, block_size, num_blocks, a.scale_log2, sink, status, s);
+    if (rc != B200_ERR_UNSUPPORTED) return rc;
+  }
   if (SIGM) a.scale_log2 = scale;      // the sigmoid of the generic kernel takes natural exponents
   dim3 grid(batch, num_q_heads);
   if (dtype == B200_DTYPE_F32)

@@ -1,5 +1,5 @@
-"""fp32 attention at head sizes 32 / 64 / 128: the tiled prompt kernel against the general kernel,
-which takes the same calls when the output does not start on a 16-byte boundary, over every form that both accept.
+"""fp32 attention at head sizes 32 / 64 / 128: the tiled prompt kernel and the clustered decode kernel against the general kernels,
+which take the same calls when the output does not start on a 16-byte boundary, over every form that both accept.
 
 Bound: both sides add at most a few thousand fp32 products and weights below one, so they differ by far less than the 2e-5 that
 fp32 kernels are held to against the oracle."""
@@ -75,3 +75,43 @@ def test_values_a_row_does_not_see_stay_out_of_it():
     for lo, hi, heads in ((0, 70, slice(0, 4)), (0, 80, slice(4, 8)), (100, 190, slice(0, 4)), (100, 150, slice(4, 8))):
         assert torch.equal(got[lo:hi, heads], want[lo:hi, heads])
     assert not torch.isfinite(got[70:100, :4, 3]).any() and not torch.isfinite(got[150:, 4:, 7]).any()
+
+
+# clusters of 8, 4, 2 and 1 CTAs per context follow from batch x heads and the length of the block table
+@pytest.mark.parametrize("page", [1, 16, 48])
+@pytest.mark.parametrize("Hq,Hkv,D,lens", [
+    (16, 4, 64, [700]), (4, 4, 32, [1, 0, 7, 8, 9, 300]), (6, 2, 128, [33, 500, 16]), (32, 8, 128, [100, 900] * 8),
+    (16, 4, 64, [2, 0, *range(1, 130, 2)]), (8, 1, 64, [63, 64, 65] * 40), (3, 1, 32, [400] * 300)])
+def test_decode(page, Hq, Hkv, D, lens):
+    from llm_from_scratch_b200 import ops
+    case = deal_blocks(lens, page, np.random.default_rng(1), pad_blocks=2)
+    kc, vc = _randn(9, case.num_blocks, page, Hkv, D), _randn(10, case.num_blocks, page, Hkv, D)
+    q, tables, ctx = _randn(11, len(lens), Hq, D), torch.from_numpy(case.block_tables).cuda(), torch.from_numpy(case.context_lens).cuda()
+    for sink in (None, _randn(12, Hq)):
+        args = (q, kc, vc, tables, ctx, D ** -0.5)
+        want = ops.paged_decode_gqa(*args, out=_off_boundary(q.shape), sink=sink)
+        _same(ops.paged_decode_gqa(*args, sink=sink), want)
+    ops.check_status()
+    tables[0, 0] = case.num_blocks + 3
+    want = ops.paged_decode_gqa(*args, out=_off_boundary(q.shape))
+    assert ops.read_status_code() != 0
+    _same(ops.paged_decode_gqa(*args), want)
+    assert ops.read_status_code() != 0
+
+
+def test_decode_calls_share_nothing():
+    """Two streams, each with calls of its own in flight, give what one gives alone."""
+    from llm_from_scratch_b200 import ops
+    case = deal_blocks([900, 20, 400], 16, np.random.default_rng(2))
+    kc, vc = _randn(13, case.num_blocks, 16, 4, 64), _randn(14, case.num_blocks, 16, 4, 64)
+    tables, ctx = torch.from_numpy(case.block_tables).cuda(), torch.from_numpy(case.context_lens).cuda()
+    qs = [_randn(15 + i, 3, 16, 64) for i in range(2)]
+    want = [ops.paged_decode_gqa(q, kc, vc, tables, ctx, 0.125) for q in qs]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in qs], [[], []]
+    for _ in range(20):
+        for i, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                got[i].append(ops.paged_decode_gqa(qs[i], kc, vc, tables, ctx, 0.125))
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, w) for outs, w in zip(got, want) for g in outs)
