@@ -19,39 +19,10 @@
 //                          columns of the state in registers and walks the tokens; q / f / k / v of 16 tokens at a
 //                          time sit in shared memory as fp32, the RG threads of a column reduce their part of o by
 //                          shuffles, and 16 tokens of outputs are normed together.
-#include "sequences.cuh"
+#include "recurrence_common.cuh"
 
 namespace b200 {
 namespace {
-
-struct RecArgs {
-  const void* q;
-  const void* f;
-  const void* v;
-  int64_t stride;            // elements between tokens, the same for q / f / v (views of one projection)
-  const float* f_bias;       // [H, dk]
-  const float* lower;        // [H, dk]
-  const float* norm_w;       // [dv]
-  float eps;
-  float* state;              // [slots, H, dk, dv]
-  const int64_t* slots;      // [n], < 0: skip the sequence
-  int64_t num_slots;
-  const int32_t* cu_q;       // [n + 1], or null: one token per sequence
-  const int32_t* cu_k;       // [n + 1] with cu_q
-  const int64_t* ctx_lens;   // [n] without cu_q: context length including the new token
-  void* out;                 // [T, H, dv]
-  int H, dk, dv;
-  int32_t* status;
-};
-
-// forget gate and write gate of one channel
-__device__ __forceinline__ void gates(float z, float lower, float* f, float* k) {
-  const float open = 1.f - lower;
-  float s, n;
-  sigmoids(z, &s, &n);
-  *f = lower + open * s;
-  *k = open * n;
-}
 
 constexpr int kStepThreads = 256;
 
@@ -159,13 +130,6 @@ int launch_step(const RecArgs& a, int n, bool vec, cudaStream_t s) {
 // Segmented scan
 // ---------------------------------------------------------------------------------------------
 constexpr int kBlockTokens = 16;     // tokens staged at a time
-
-struct ScanArgs {
-  float* seg_state;          // [segments, H, dk, dv]  pass 1: P, after pass 2: entry state
-  float* seg_decay;          // [segments, H, dk]      pass 1: D
-  int n, seg_len;
-  bool async;                // 16-byte copies are possible
-};
 
 // RG: threads that share a column group
 template <typename T, int R, int C, int RG, bool LOCAL>
@@ -406,6 +370,16 @@ __global__ void __launch_bounds__(256) recurrence_chain_kernel(const RecArgs a, 
   *reinterpret_cast<float4*>(st) = S;
 }
 
+}  // namespace
+
+int recurrence_chain_launch(const RecArgs& a, const ScanArgs& sc, cudaStream_t s) {
+  const int64_t units = static_cast<int64_t>(a.dk) * a.dv / 4;
+  recurrence_chain_kernel<<<dim3(static_cast<unsigned>((units + 255) / 256), a.H, sc.n), 256, 0, s>>>(a, sc);
+  return launch_result();
+}
+
+namespace {
+
 // sizes the scan takes: columns of all threads of a CTA, rows in registers
 inline bool scan_shape(int dk, int dv) { return dv % 4 == 0 && ((dk <= 128 && dv <= 256) || (dk <= 256 && dv <= 128)); }
 
@@ -430,8 +404,8 @@ int launch_scan(const RecArgs& a, const ScanArgs& sc, int64_t segments, bool cha
   const dim3 grid(static_cast<unsigned>(segments), a.H);
   if (chained) {
     local<<<grid, threads, smem_local, s>>>(a, sc);
-    const int64_t units = static_cast<int64_t>(a.dk) * a.dv / 4;
-    recurrence_chain_kernel<<<dim3(static_cast<unsigned>((units + 255) / 256), a.H, sc.n), 256, 0, s>>>(a, sc);
+    const int rc = recurrence_chain_launch(a, sc, s);
+    if (rc != B200_OK) return rc;
   }
   full<<<grid, threads, smem_full, s>>>(a, sc);
   return launch_result();
@@ -483,6 +457,11 @@ extern "C" int b200_gated_recurrence(const void* q, const void* f, const void* v
     const int64_t es = dtype == B200_DTYPE_F32 ? 4 : 2;
     sc.async = dim_k * es % 16 == 0 && dim_v * es % 16 == 0 && token_stride * es % 16 == 0 && aligned16(q) &&
                aligned16(f) && aligned16(v);
+    // bf16 and heads of 64 or 128 run on tensor cores: 8 x 1,024 tokens x 16 heads of 128 227 us against 786 us
+    const bool chunks = dtype == B200_DTYPE_BF16 && recurrence_chunk_shape(dim_k, dim_v) && sc.async && aligned16(f_bias) &&
+                        aligned16(lower) && aligned16(norm_w) && aligned16(out);
+    // never shorter than the scan's: the workspace is sized for those
+    if (chunks) sc.seg_len = max(sc.seg_len, recurrence_chunk_seg_len(total_tokens, max_seqlen_q, num_heads));
     const int64_t segments = total_tokens / sc.seg_len + num_seqs;
     const bool chained = max_seqlen_q > sc.seg_len;
     if (chained) {
@@ -492,6 +471,7 @@ extern "C" int b200_gated_recurrence(const void* q, const void* f, const void* v
       sc.seg_state = static_cast<float*>(workspace);
       sc.seg_decay = sc.seg_state + static_cast<size_t>(segments) * num_heads * dim_k * dim_v;
     }
+    if (chunks) return recurrence_chunk_launch(a, sc, segments, chained, s);
     return dtype == B200_DTYPE_F32 ? dispatch_scan<float>(a, sc, segments, chained, s)
                                    : dispatch_scan<__nv_bfloat16>(a, sc, segments, chained, s);
   }

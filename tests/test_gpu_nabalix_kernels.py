@@ -229,6 +229,41 @@ def test_gated_recurrence_in_portions_and_steps(H, dk, dv, dtype, tol):
     assert (state[[1, 3]] == 7.0).all()
 
 
+@pytest.mark.parametrize("H,d", [(3, 64), (2, 128), (16, 64), (9, 128)])
+@pytest.mark.parametrize("lens", [[700, 1, 16, 17], [32, 15, 1, 31, 2], [129, 128, 127]])
+def test_gated_recurrence_blocks_of_sixteen_tokens(H, d, lens):
+    """Whole and cut sequences around the edges of a block and of a segment, some of them continued; channels that forget
+    everything within a token or nothing at all.  State: what a token wrote is multiplied by one fp32 gate per later token, each
+    with a rounding of the gate and one of the product (2^-24 together), on top of the 24-bit operands and the sums of a block
+    (16 roundings): (tokens + 16) 2^-24."""
+    from llm_from_scratch_b200 import ops
+    eps, n, w = 1e-5, len(lens), H * d
+    g = gen(d + H)
+    r = lambda *s: torch.randn(*s, generator=g)
+    fb, lower, nw = r(w) * 3, torch.rand(w, generator=g), r(d)
+    lower[::5] = 0
+    fb[1::7], lower[1::7] = -60.0, 0
+    fb[2::7] = 60.0
+    proj, before = r(sum(lens), 3 * w).bfloat16() * 2, r(n, H, d, d)
+    old = [0 if i % 2 else 5 for i in range(n)]                  # tokens of earlier portions
+    state = torch.full((n + 1, H, d, d), 7.0)
+    slots = torch.tensor([(i * 2 + 1) % (n + 1) for i in range(n)]) if n % 2 == 0 else torch.arange(n)
+    state[slots] = before
+    cu = lambda x: torch.tensor(np.concatenate([[0], np.cumsum(x)]), dtype=torch.int32).cuda()
+    x, got = proj.cuda(), state.cuda()
+    y = ops.gated_recurrence(x[:, :w], x[:, w:2 * w], x[:, 2 * w:], fb.cuda(), lower.cuda(), nw.cuda(), eps, got, slots.cuda(),
+                             cu_seqlens_q=cu(lens), cu_seqlens_k=cu([a + b for a, b in zip(lens, old)]), max_seqlen_q=max(lens))
+    ops.check_status()
+    for i, (p, o) in enumerate(zip(proj.double().split(lens), y.split(lens))):
+        f = orc.forget_gate(p[:, w:2 * w], fb.double(), lower.double()).view(-1, H, d)
+        want, S = orc.gated_recurrence(orc.silu(p[:, :w]).view(-1, H, d), f, p[:, 2 * w:].reshape(-1, H, d),
+                                       before[i].double() if old[i] else None)
+        assert rel(o, orc.norm_plain(want, nw.double(), eps).reshape(len(p), -1)) < 4e-3          # bf16 outputs: half a step is 2^-9
+        assert rel(got[slots[i]], S) < (len(p) + 16) * 2.0 ** -24
+    free = [s for s in range(n + 1) if s not in slots.tolist()]
+    assert (got[free] == 7.0).all()
+
+
 def test_store_kv_rows_of_unequal_widths():
     from llm_from_scratch_b200 import ops
     for wk, wv, dtype in ((64, 96, torch.bfloat16), (21, 10, torch.bfloat16), (12, 20, torch.float32), (3, 5, torch.float32)):
