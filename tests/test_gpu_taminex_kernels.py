@@ -358,6 +358,23 @@ def test_chunked_delta_rule_keeps_fp32_accuracy(slow):
     assert (y.float() != z.float()).float().mean() < 0.01            # outputs differ in a bf16 rounding here and there
 
 
+@pytest.mark.parametrize("dv", [16, 48, 64])
+@pytest.mark.parametrize("lens", [[1], [63, 64, 65], [128, 2, 193], [1, 129]])
+def test_chunks_of_two_warp_groups_against_the_walk(dv, lens):
+    """Key heads of 64 channels: chunk edges, and what follows a sequence's last rows is not its own: the next sequence holds
+    infinities.  Equal activations on both sides: the states differ by fp32 roundings, outputs by a bf16 rounding here and there."""
+    rows = [*lens, 40]
+    d, e = (Delta(4, 2, 64, dv, 4, rows, torch.bfloat16, seed=dv + len(lens)) for _ in range(2))
+    for x in (d, e):
+        x.proj[-1][:, :4 * 64 + 4 * dv] = float("inf")
+    ranges = [(i, 0, n) for i, n in enumerate(rows)]
+    got, want = d.step(ranges), e.step(ranges, general=True)
+    for i, (y, z) in enumerate(zip(got[:-1], want[:-1])):
+        assert torch.isfinite(y.float()).all()
+        assert (y.float() != z.float()).float().mean() < 0.01
+        close(d.state[d.slots[i]], e.state[e.slots[i]].cpu(), STATE_TOL[torch.bfloat16])
+
+
 def test_delta_rule_with_strong_decays_and_large_inputs():
     d = Delta(4, 2, 64, 64, 4, [130, 64], torch.bfloat16, seed=2, scale=12.0)
     for y, w in zip(d.step([(0, 0, 130), (1, 0, 64)]), d.want):
