@@ -88,7 +88,14 @@ struct Args2 {
   const __nv_bfloat16* gate;   // [tokens, Hq] or null (SIGM kernels)
   int64_t gate_stride;
   int32_t* status;
+  bool beside_store;     // the launch before this one is the scatter of its keys and values
 };
+
+// Started beside the launch before it (the step's scatter of keys and values, which nothing here reads): a CTA does not end
+// before that has ended, so that what follows in the stream finds its rows.  Returns at once in an ordinary launch.
+__device__ __forceinline__ void end_behind_store(int tid) {
+  if (tid == 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
 
 template <int DQK, int DV, bool TAIL, bool WINDOW, bool SIGM>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -108,7 +115,7 @@ prefill_umma2_kernel(const Args2 a, const __grid_constant__ CUtensorMap tm_q, co
   const int head = blockIdx.x;
   int seq, tile;
   if (a.plan) {                                  // grid (head, tile-list slot)
-    if (static_cast<int>(blockIdx.y) >= a.plan[0]) return;
+    if (static_cast<int>(blockIdx.y) >= a.plan[0]) return end_behind_store(tid);
     const uint32_t entry = static_cast<uint32_t>(a.plan[kPlanHeader + blockIdx.y]);
     seq = entry >> 16;
     tile = entry & 0xffffu;
@@ -119,7 +126,7 @@ prefill_umma2_kernel(const Args2 a, const __grid_constant__ CUtensorMap tm_q, co
   const int q0 = a.cu_q[seq], q_len = a.cu_q[seq + 1] - q0;
   int k0 = a.cu_k[seq], k_len = a.cu_k[seq + 1] - k0;
   const int m0 = tile * ROWS;
-  if (m0 >= q_len) return;                       // uniform over the CTA, before any barrier / allocation
+  if (m0 >= q_len) return end_behind_store(tid);      // uniform over the CTA, before any barrier / allocation
   int off = k_len - q_len;
   int skip = 0;                                  // keys ahead of the walk
   // first key that the query sees whose own key is number i, in keys of the walk (may be negative)
@@ -515,6 +522,7 @@ prefill_umma2_kernel(const Args2 a, const __grid_constant__ CUtensorMap tm_q, co
   umma::fence_before_sync();
   __syncthreads();
   if (warp == 2) umma::tmem_dealloc(tmem, L::TCOLS);
+  end_behind_store(tid);
 }
 
 }  // namespace
@@ -572,8 +580,17 @@ int launch2(const Args2& a, const CUtensorMap& tq, const CUtensorMap& tk, const 
       return B200_ERR_LAUNCH;
     configured[dev] = true;
   }
-  kern<<<grid, kThreads, L::SMEM, s>>>(a, tq, tk, tkt, tv);
-  return launch_result();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = L::SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = a.beside_store ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, a, tq, tk, tkt, tv) == cudaSuccess ? launch_result() : B200_ERR_LAUNCH;
 }
 
 }  // namespace
@@ -595,7 +612,8 @@ int prefill_umma2_launch(const void* q, const void* k, const void* v, void* out,
                          int64_t v_stride, int64_t total_q, int64_t total_k, const int32_t* cu_q,
                          const int32_t* cu_k, int num_seqs, int max_seqlen_q, int Hq, int Hkv, int Dqk, int Dv,
                          float scale, const int32_t* plan, int plan_tile_rows, int plan_capacity, int32_t* status,
-                         cudaStream_t s, const void* k_tail, int64_t k_tail_stride, int tail, const float* sink, int window) {
+                         cudaStream_t s, const void* k_tail, int64_t k_tail_stride, int tail, const float* sink, int window,
+                         bool beside_store) {
   if (prefill_umma2_tile_rows(Hq, Hkv, Dqk, Dv) == 0) return B200_ERR_UNSUPPORTED;
   if (tail != 0 && (tail != 64 || Dqk != 192 || k_tail == nullptr)) return B200_ERR_UNSUPPORTED;
   if (!(scale > 0.f)) return B200_ERR_UNSUPPORTED;   // the row maximum is taken before scaling
@@ -615,6 +633,7 @@ int prefill_umma2_launch(const void* q, const void* k, const void* v, void* out,
   a.scale_log2 = scale * 1.4426950408889634f;
   a.sink = sink;
   a.window = window;
+  a.beside_store = beside_store;
   a.status = status;
   CUtensorMap tq, tk, tkt, tv;
   memset(&tq, 0, sizeof(tq));

@@ -58,7 +58,14 @@ struct Args4 {
   float scale_log2;
   const float* sink;     // [Hq] or null
   int32_t* status;
+  bool beside_store;     // the launch before this one is the scatter of its keys and values
 };
+
+// Started beside the launch before it (the step's scatter of keys and values, which nothing here reads): a CTA does not end
+// before that has ended, so that what follows in the stream finds its rows.  Returns at once in an ordinary launch.
+__device__ __forceinline__ void end_behind_store(int tid) {
+  if (tid == 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
 
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_umma4_kernel(const Args4 a, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -76,7 +83,7 @@ prefill_umma4_kernel(const Args4 a, const __grid_constant__ CUtensorMap tm_q, co
   const int kvh = head0 / G;
   int seq, tile;
   if (a.plan) {                                  // grid (head group, tile-list slot)
-    if (static_cast<int>(blockIdx.y) >= a.plan[0]) return;
+    if (static_cast<int>(blockIdx.y) >= a.plan[0]) return end_behind_store(tid);
     const uint32_t entry = static_cast<uint32_t>(a.plan[kPlanHeader + blockIdx.y]);
     seq = entry >> 16;
     tile = entry & 0xffffu;
@@ -87,7 +94,7 @@ prefill_umma4_kernel(const Args4 a, const __grid_constant__ CUtensorMap tm_q, co
   const int q0 = a.cu_q[seq], q_len = a.cu_q[seq + 1] - q0;
   const int k0 = a.cu_k[seq], k_len = a.cu_k[seq + 1] - k0;
   const int m0 = tile * BM;
-  if (m0 >= q_len) return;                       // uniform over the CTA, before any barrier / allocation
+  if (m0 >= q_len) return end_behind_store(tid);      // uniform over the CTA, before any barrier / allocation
   const int off = k_len - q_len;
   const int rows = min(BM, q_len - m0);
   int kmax = off + m0 + rows;                    // keys visible to the last row of the tile
@@ -338,6 +345,7 @@ prefill_umma4_kernel(const Args4 a, const __grid_constant__ CUtensorMap tm_q, co
   umma::fence_before_sync();
   __syncthreads();
   if (warp == 2) umma::tmem_dealloc(tmem, TCOLS);
+  end_behind_store(tid);
 }
 
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -391,7 +399,7 @@ int prefill_umma4_launch(const void* q, const void* k, const void* v, void* out,
                          int64_t v_stride, int64_t total_q, int64_t total_k, const int32_t* cu_q,
                          const int32_t* cu_k, int num_seqs, int max_seqlen_q, int Hq, int Hkv, int Dqk, int Dv,
                          float scale, const int32_t* plan, int plan_tile_rows, int plan_capacity, int32_t* status,
-                         cudaStream_t s, const float* sink) {
+                         cudaStream_t s, const float* sink, bool beside_store) {
   if (prefill_umma4_tile_rows(Hq, Hkv, Dqk, Dv) == 0) return B200_ERR_UNSUPPORTED;
   if (!(scale > 0.f)) return B200_ERR_UNSUPPORTED;   // the row maximum is taken before scaling
   const int ntiles = (max_seqlen_q + BM - 1) / BM;
@@ -408,6 +416,7 @@ int prefill_umma4_launch(const void* q, const void* k, const void* v, void* out,
   a.plan = (plan != nullptr && plan_tile_rows == BM && plan_capacity > 0 && plan_capacity <= 65535) ? plan : nullptr;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.sink = sink;
+  a.beside_store = beside_store;
   a.status = status;
   CUtensorMap tq, tk, tv;
   memset(&tq, 0, sizeof(tq));
@@ -428,8 +437,17 @@ int prefill_umma4_launch(const void* q, const void* k, const void* v, void* out,
   }
   dim3 grid(Hq / NP, num_seqs, ntiles);
   if (a.plan) grid = dim3(Hq / NP, plan_capacity, 1);
-  prefill_umma4_kernel<<<grid, kThreads, SMEM, s>>>(a, tq, tk, tv);
-  return launch_result();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = a.beside_store ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, prefill_umma4_kernel, a, tq, tk, tv) == cudaSuccess ? launch_result() : B200_ERR_LAUNCH;
 }
 
 }  // namespace b200

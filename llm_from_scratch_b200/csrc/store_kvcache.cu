@@ -21,6 +21,8 @@ store_kvcache_vec16(const uint4* __restrict__ k, const uint4* __restrict__ v, in
                     int64_t v_stride, uint4* __restrict__ kc, uint4* __restrict__ vc,
                     const int64_t* __restrict__ slots, int64_t total, int cpr, int64_t num_slots,
                     int32_t* status) {
+  // a prompt's attention over packed keys may be placed beside this grid (it ends behind it)
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   const int64_t step = static_cast<int64_t>(gridDim.x) * kThreads;
   for (int64_t base = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x; base < total;
        base += step * kUnroll) {
