@@ -49,14 +49,14 @@ FAMILY_SOURCES = {
     "Nabalix": ("api", "host_path", "decode_advance", "sampler", "moe_gemm", "moe_gemm_rows", "grouped_linear", "store_kvcache", "prefill_plan", "streams",
                 "talking_attention", "talking_attention_mma", "talking_decode_mma", "gated_recurrence", "recurrence_chunk"),
     "Taminex": ("api", "host_path", "decode_advance", "sampler", "moe_gemm", "moe_gemm_rows", "grouped_linear", "store_kvcache", "prefill_plan",
-                "prefill_varlen", "prefill_f32", "prefill_mma", "prefill_umma", "prefill_umma2", "prefill_umma4", "paged_decode", "decode_f32", "mla_decode",
+                "prefill_varlen", "prefill_f32", "prefill_mma", "prefill_umma", "prefill_umma2", "prefill_umma4", "paged_decode", "decode_cluster", "decode_f32", "mla_decode",
                 "mla_decode_mma", "residual_norm", "head_norm_rope", "latent_rows", "activations", "delta_rule", "delta_chunk"),
     "Meresun": ("api", "host_path", "decode_advance", "sampler", "moe_gemm", "moe_gemm_rows", "grouped_linear", "moe_group_route",
                 "store_kvcache", "prefill_plan", "prefill_varlen", "prefill_f32", "prefill_mma", "prefill_umma", "prefill_umma2", "prefill_umma4",
-                "paged_decode", "decode_f32", "mla_decode", "mla_decode_mma", "residual_norm", "gated_residual", "latent_rows", "activations"),
+                "paged_decode", "decode_cluster", "decode_f32", "mla_decode", "mla_decode_mma", "residual_norm", "gated_residual", "latent_rows", "activations"),
     "Sodonex": ("api", "host_path", "decode_advance", "sampler", "moe_gemm", "moe_gemm_rows", "grouped_linear", "moe_group_route",
                 "store_kvcache", "prefill_plan", "prefill_varlen", "prefill_f32", "prefill_mma", "prefill_umma", "prefill_umma2", "prefill_umma4",
-                "paged_decode", "decode_f32", "latent_rows", "activations", "shift_residual", "conv_norm_rope"),
+                "paged_decode", "decode_cluster", "decode_f32", "latent_rows", "activations", "shift_residual", "conv_norm_rope"),
 }
 
 

@@ -27,6 +27,8 @@
 // V^T . P^T, so each K/V byte is read from HBM exactly once and used for all G heads.  Softmax is
 // the online form in fp32 in the log2 domain; column statistics are reduced with warp shuffles.
 //
+// Head size 128 runs decode_cluster.cu where the stream is not the faster form (the rule stands there).
+//
 // Generic path (any dtype / head_dim <= 256 / block size): one CTA per (sequence, query head),
 // fp32 FMA arithmetic.  fp32 at head sizes 32 / 64 / 128 runs decode_f32.cu instead.
 //
@@ -826,6 +828,10 @@ namespace b200 {
 int decode_f32_launch(const void* q, const void* kc, const void* vc, void* out, const int32_t* bt, int64_t bt_stride,
                       const int64_t* lens, int batch, int Hq, int Hkv, int D, int Dv, int bs, int64_t num_blocks,
                       float scale_log2, const float* sink, int32_t* status, cudaStream_t s);
+// bf16, small batches (decode_cluster.cu)
+int decode_cluster_launch(const void* q, const void* kc, const void* vc, void* out, const int32_t* bt, int64_t bt_stride,
+                          const int64_t* lens, int batch, int Hq, int Hkv, int D, int sub, int64_t num_blocks, float scale_log2,
+                          const float* sink, int32_t* status, cudaStream_t s);
 
 namespace {
 // what the sigmoid form has in addition
@@ -889,6 +895,11 @@ static int paged_decode(const void* q, const void* k_cache, const void* v_cache,
                                                               head_dim, dtype);
     if (!workspace || workspace_bytes < need) return B200_ERR_WORKSPACE;
     if (reinterpret_cast<uintptr_t>(workspace) & 255u) return B200_ERR_ALIGN;
+    if constexpr (!SIGM) {       // clusters of CTAs where they are the faster form: no scratch is touched
+      const int rc = decode_cluster_launch(q, k_cache, v_cache, out, block_tables, bt_stride, context_lens, batch, num_q_heads,
+                                           num_kv_heads, head_dim, a.sub, num_blocks, a.scale_log2, sink, status, s);
+      if (rc != B200_ERR_UNSUPPORTED) return rc;
+    }
     const size_t grid = static_cast<size_t>(sms) * pl.ctas_per_sm;
     uint8_t* w = static_cast<uint8_t*>(workspace);
     // Which merge: inside the launch for small batches, where a step is a chain of short kernels and one launch

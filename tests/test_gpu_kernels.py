@@ -154,6 +154,31 @@ def test_paged_decode_bf16_long_sequence_split_across_ctas():
     assert_close(got, want, torch.bfloat16)
 
 
+@pytest.mark.parametrize("Hq,Hkv,D,bs", [(32, 8, 128, 64), (12, 1, 128, 256), (6, 3, 128, 16), (16, 1, 128, 32)])
+@pytest.mark.parametrize("lens", [[1], [700], [16, 64, 65, 128, 129], [511, 0, 513, 2048, 15], [1030] * 40])
+@pytest.mark.parametrize("sink", [False, True])
+def test_decode_in_clusters_and_in_one_stream(Hq, Hkv, D, bs, lens, sink):
+    """Both bf16 forms on the same contexts: block tables as wide as the contexts need go to clusters of CTAs, tables that allow
+    far longer contexts to the streaming kernel.  Contexts around the blocks, warps and CTAs that share them; empty ones;
+    block numbers behind a context are never read."""
+    ops, orc = _ops(), _oracle()
+    case, q, kc, vc = _decode_case(lens, Hq, Hkv, D, bs, torch.bfloat16, seed=D + len(lens))
+    s = _randn((Hq,), 5, torch.float32) if sink else None
+    want = orc.paged_decode_gqa(q, kc, vc, case.block_tables, case.context_lens, D ** -0.5)
+    if sink:        # the sum of a row is that of its weights without sinks
+        scores = [torch.einsum("hd,nhd->hn", q[i].float(), kc[torch.from_numpy(case.block_tables[i, :-(-n // bs)]).long()].flatten(0, 1)[:n]
+                               .float().repeat_interleave(Hq // Hkv, 1)) * D ** -0.5 for i, n in enumerate(lens)]
+        lse = torch.stack([torch.logsumexp(x, -1) if x.shape[1] else torch.full((Hq,), float("inf")) for x in scores])
+        want = want * torch.sigmoid(lse - s)[:, :, None]
+    wide = np.full((len(lens), 8 * 4096 // bs * 2 + 8), 2 ** 30, dtype=np.int32)
+    wide[:, :case.block_tables.shape[1]] = case.block_tables
+    for table in (case.block_tables, wide):
+        got = ops.paged_decode_gqa(q.cuda(), kc.cuda(), vc.cuda(), torch.from_numpy(table).cuda(),
+                                   torch.from_numpy(case.context_lens).cuda(), D ** -0.5, sink=None if s is None else s.cuda())
+        ops.check_status()
+        assert_close(got, want, torch.bfloat16)
+
+
 def test_paged_decode_bf16_single_short_sequence_and_stale_table_entries():
     # entries past ceil(len/16) hold stale ids outside the pool: they must never be read
     case, q, kc, vc = _decode_case([20], 32, 8, 128, 16, torch.bfloat16, seed=3)
