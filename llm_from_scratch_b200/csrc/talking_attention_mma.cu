@@ -15,6 +15,11 @@
 // accumulator to the exponential.  The running maximum is lazy: a row keeps the reference maximum of an earlier tile
 // until a score exceeds it by 2^kSlack, so the ordinary tile needs no reduction over lanes; the maximum only has to
 // keep the exponentials in range.
+//
+// What bounds it: latency and issue slots of a tile, 16 warps per SM (tensor pipe 20 %, data pipe of shared memory 43 %).  With
+// the number of heads known to the compiler (plane offsets become immediates, nothing spills) and the block table read a tile
+// ahead of the rows, 8 prompts of 1,024 tokens x 16 heads of 128 take 345 us instead of 402, 32 heads of 128 1,097 instead of
+// 1,188; results are the same bits.
 #include <string.h>
 
 #include "talking_attention.cuh"
@@ -55,14 +60,14 @@ __device__ __forceinline__ float capped(float x, float k, float cap, float two_c
 }
 
 // HP: heads padded; NW: warps; MAXC: value columns per CTA in units of 16; MODE: 0 any constants, 1 soft cap and bias table
-// present, 2 also H == HP, 3 as 1 with the mix on tensor cores (a talk matrix of bf16 values); q_smem: the query rows are staged in shared memory (else their fragments are read from global memory)
+// present, 2 also H == HP, 3 as 1 with the mix on tensor cores (a talk matrix of bf16 values), 4 also H == HP; q_smem: the query rows are staged in shared memory (else their fragments are read from global memory)
 // PAIR: tiles of eight queries, and the sixteen rows of a warp's MMA tile are those of two neighbouring heads that
 // share a key head: half the accumulators per head, so that many or wide heads fit
 template <int HP, int NW, int MAXC, int MINB, int MODE, bool PAIR>
 __global__ void __launch_bounds__(NW * 32, MINB)
 talking_prefill_kernel(const TalkArgs a, const __grid_constant__ MixParam<HP> mp, const int layout) {
   constexpr int BQ = PAIR ? kTalkTileRows / 2 : kTalkTileRows, kPlane = plane_floats(BQ);
-  static_assert(!PAIR || (MODE == 3 && HP == 2 * NW), "a pair of heads per warp");
+  static_assert(!PAIR || (MODE >= 3 && HP == 2 * NW), "a pair of heads per warp");
   constexpr bool kHalfRow = PAIR && NW == 16;          // two warps share a query row of the mix
   constexpr int HPW = PAIR ? 1 : HP / NW, kThreads = NW * 32, kTpr = kThreads / BK;    // kTpr: threads that load one key row
   const bool q_smem = layout & kQueryInSmem, two_scores = layout & kTwoScores;
@@ -70,12 +75,12 @@ talking_prefill_kernel(const TalkArgs a, const __grid_constant__ MixParam<HP> mp
   __shared__ __align__(16) float s_ref[BQ * HP];     // reference maximum (log2 domain) per (row, head)
   __shared__ float s_cor[2][BQ * HP];  // by tile parity: factor for accumulators and sums, 1 unless the flag is set
   constexpr int kTalkRow = HP / 2 + 4;           // words per row of the matrix, padded against bank conflicts
-  __shared__ uint32_t s_talk[MODE == 3 ? HP * kTalkRow : 1];
+  __shared__ uint32_t s_talk[MODE >= 3 ? HP * kTalkRow : 1];
   __shared__ float s_top[kHalfRow ? 2 * BQ * HP : 1];
   __shared__ int s_up[kHalfRow ? BQ : 1];
   __shared__ int s_flag[2], s_seq, s_tile;       // flag (by tile parity): some reference moved
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
-  const int H = MODE == 2 ? HP : a.H, G = a.Hkv, Gs = H / G, dk = a.dk;
+  const int H = MODE == 2 || MODE == 4 ? HP : a.H, G = a.Hkv, Gs = H / G, dk = a.dk;
   const int dvc = a.dv / gridDim.y, dv0 = blockIdx.y * dvc, nc = dvc / 16;
 
   // ---- which (sequence, tile): from the step's tile list (heaviest first), or numbered sequence by sequence ----
@@ -187,7 +192,7 @@ talking_prefill_kernel(const TalkArgs a, const __grid_constant__ MixParam<HP> mp
       cp_async16(sQ + ((h * BQ + r) * strQ + cc * 8) * 2, src, r < rows ? 16 : 0);
     }
   }
-  int64_t next_row = tile_row(0);
+  int64_t next_row = tile_row(0), then_row = tile_row(1);      // the table is read a tile ahead of the rows
   load_rows(next_row, a.kc, dk, 0, dk, sK, strK);
   cp_async_commit();
   load_rows(next_row, a.vc, a.dv, dv0, dvc, sV, strV);
@@ -200,7 +205,7 @@ talking_prefill_kernel(const TalkArgs a, const __grid_constant__ MixParam<HP> mp
   }
   if (tid < 2) s_flag[tid] = 0;
   if (kHalfRow && tid < BQ) s_up[tid] = 0;
-  if constexpr (MODE == 3)
+  if constexpr (MODE >= 3)
     for (int i = tid; i < HP * HP / 2; i += kThreads) s_talk[i / (HP / 2) * kTalkRow + i % (HP / 2)] = mp.tb[i];
 
   float o[HPW][2 * MAXC][4], l[HPW][2];
@@ -407,8 +412,9 @@ talking_prefill_kernel(const TalkArgs a, const __grid_constant__ MixParam<HP> mp
   cp_async_wait<0>();
   __syncthreads();
   if (ntiles > 1) {
-    next_row = tile_row(1);
+    next_row = then_row;
     load_rows(next_row, a.kc, dk, 0, dk, sK, strK);
+    then_row = tile_row(2);
   }
   cp_async_commit();
 
@@ -417,7 +423,7 @@ talking_prefill_kernel(const TalkArgs a, const __grid_constant__ MixParam<HP> mp
     const int buf = two_scores ? t & 1 : 0;
     float* S = S0 + buf * (H * kPlane);
     // ---- mix ----
-    if constexpr (MODE == 3) mix_mma(S, t);
+    if constexpr (MODE >= 3) mix_mma(S, t);
     else
 #pragma unroll 1
     for (int r = warp; r < rows; r += NW) {
@@ -547,9 +553,10 @@ talking_prefill_kernel(const TalkArgs a, const __grid_constant__ MixParam<HP> mp
     __syncthreads();
     if (t + 1 < ntiles) load_rows(next_row, a.vc, a.dv, dv0, dvc, sV, strV);
     if (t + 2 < ntiles) {
-      next_row = tile_row(t + 2);
+      next_row = then_row;
       load_rows(next_row, a.kc, dk, 0, dk, sK, strK);
       load_bias(t + 2);
+      then_row = tile_row(t + 3);
     }
     cp_async_commit();
   }
@@ -638,7 +645,8 @@ int launch_prefill(const TalkArgs& a, int chunks, size_t smem, int layout, cudaS
   if (a.cap > 0.f && a.window > 0 && a.bias_len >= a.window) {
     if constexpr (HP >= 16) {
       if (exact_in_bf16(a.talk_host, a.H * a.H))
-        return launch_prefill<HP, NW, MAXC, MINB, 3>(a, chunks, smem, layout, s);
+        return a.H == HP ? launch_prefill<HP, NW, MAXC, MINB, 4>(a, chunks, smem, layout, s)
+                         : launch_prefill<HP, NW, MAXC, MINB, 3>(a, chunks, smem, layout, s);
     } else if (a.H == HP) {
       return launch_prefill<HP, NW, MAXC, MINB, 2>(a, chunks, smem, layout, s);
     }
@@ -667,7 +675,8 @@ int talking_prefill_mma_launch(const TalkArgs& a, cudaStream_t s) {
   if (tensor_mix && a.H > 16 && (a.H / a.Hkv) % 2 == 0 && a.dv <= 128) {     // many heads: pairs of heads on eight queries
     for (int l : {kQueryInSmem | kTwoScores, +kTwoScores, +kQueryInSmem, 0}) {
       const size_t smem = smem_of(kTalkTileRows / 2, a.dv, l);
-      if (smem <= 212 * 1024) return launch_prefill<32, 16, 8, 1, 3, true>(a, 1, smem, l, s);
+      if (smem <= 212 * 1024)
+        return a.H == 32 ? launch_prefill<32, 16, 8, 1, 4, true>(a, 1, smem, l, s) : launch_prefill<32, 16, 8, 1, 3, true>(a, 1, smem, l, s);
     }
   }
   for (int chunks = 1; chunks <= a.dv / 16; ++chunks) {
