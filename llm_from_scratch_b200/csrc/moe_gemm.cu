@@ -487,7 +487,7 @@ int launch(const GemmArgs& a, const CUtensorMap& tw, const CUtensorMap& tx, dim3
 
 int moe_gemm_rows_launch(const void* x, const void* w, const void* bias, void* out, const int32_t* expert_offsets,
                          int64_t num_rows, int num_experts, int dense_rows, int n_out, int k_dim, int mode, float limit,
-                         float slope, int32_t* status, cudaStream_t s);
+                         float slope, int32_t* status, bool early, cudaStream_t s);
 int grouped_linear_any_launch(const void* x, const void* w, void* out, const int32_t* expert_offsets, int64_t num_rows,
                               int num_experts, int n_out, int k_dim, int act, float limit, float slope, int32_t dtype,
                               cudaStream_t s);
@@ -526,7 +526,7 @@ int grouped_gemm(const void* x, const void* w, const void* bias, void* out, cons
   }
   // many rows per expert: the compute-bound kernel (token rows as the MMA M side, persistent CTAs)
   const int rc = moe_gemm_rows_launch(x, w, bias, out, expert_offsets, num_rows, num_experts, dense_rows, n_out, k_dim,
-                                      mode, limit, slope, status, s);
+                                      mode, limit, slope, status, early, s);
   if (rc != B200_ERR_UNSUPPORTED) return rc;
   const dim3 grid(tiles, num_experts + (dense_rows + 255) / 256);
   return launch<256, 4>(a, tw, tx, grid, early, s);

@@ -524,108 +524,115 @@ paged_decode_bf16_kernel(const DecodeArgs a) {
   cp_async_wait<0>();
 }
 
-// Merges the partial results of sequences that were cut across CTAs; zero-fills rows whose
-// context is empty.  One CTA per sequence.  Most sequences are not cut and leave at once; for the
-// others the per-head weights 2^(m_p - M) / L are computed once into shared memory, then every
-// thread sums its float4 columns over the parts with all loads of a trip independent.
+// Merges the partial results of sequences that were cut across CTAs; zero-fills rows whose context is empty.  A CTA takes one float4
+// column per thread of one sequence; most sequences are not cut and leave at once.  Bound by the chain of its loads: who was cut,
+// maxima and sums of all pieces at once into shared memory, and meanwhile the first four pieces of the column.  Sums run over
+// the pieces in their order.  (Piece after piece, with four columns per thread, the latent decode of
+// 8 x 2,000 tokens took 49 us as a whole, this form 25; 128 x 64 .. 1,024 tokens at 16/4 heads x 64 20.7 and 18.9.)
 constexpr int kCombineThreads = 256;
-constexpr int kCombineMaxParts = 8;  // parts whose weights are kept in shared memory per trip
+constexpr int kCombineAhead = 4;     // pieces of a column in flight
+// pieces whose maxima, sums and weights are held in shared memory at a time
+inline int combine_parts(int Hq) { return Hq >= 256 ? 8 : Hq >= 64 ? 16 : 32; }
 
 __global__ void __launch_bounds__(kCombineThreads)
-paged_decode_combine_kernel(const DecodeArgs a) {
-  extern __shared__ float s_w[];  // [kCombineMaxParts][Hq]
+paged_decode_combine_kernel(const DecodeArgs a, int P) {
+  extern __shared__ __align__(16) float s_w[];                         // weights [P][Hq]
+  float2* s_ml = reinterpret_cast<float2*>(s_w + P * a.Hq);            // maximum and sum [P][Hq]
+  float* s_M = reinterpret_cast<float*>(s_ml + P * a.Hq);              // [Hq]
+  float* s_inv = s_M + a.Hq;                                           // [Hq]
   // launched early (programmatic dependent of the attention kernel): everything below reads its results
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
-  const int i = blockIdx.x;
-  const int n = a.Hq * a.D;
-  __nv_bfloat16* op = static_cast<__nv_bfloat16*>(a.out) + static_cast<int64_t>(i) * n;
+  const int i = blockIdx.x, n = a.Hq * a.D, tid = threadIdx.x;
+  const int col = (blockIdx.y * kCombineThreads + tid) * 4;            // D is a multiple of 16 on this path
+  const bool in = col < n;
+  __nv_bfloat16* op = static_cast<__nv_bfloat16*>(a.out) + static_cast<int64_t>(i) * n + col;
   const int64_t len = a.lens[i];
   const int first = a.seq_info[2 * i], last = a.seq_info[2 * i + 1];
   if (len <= 0) {
-    for (int e = threadIdx.x; e < n; e += kCombineThreads) op[e] = __float2bfloat16_rn(0.f);
+    if (in)
+      for (int e = 0; e < 4; ++e) op[e] = __float2bfloat16_rn(0.f);
     return;
   }
   if (first < 0) return;
   const int np = last - first + 1;
-  auto slot_of = [&](int p) -> int64_t {
-    return static_cast<int64_t>(first + p) * 2 + (p == 0 ? 1 : 0);
+  auto slot_of = [&](int p) -> int64_t { return static_cast<int64_t>(first + p) * 2 + (p == 0 ? 1 : 0); };
+  float4 x[kCombineAhead];
+  auto load = [&](int p0) {
+#pragma unroll
+    for (int u = 0; u < kCombineAhead; ++u)
+      if (in && p0 + u < np) x[u] = __ldcg(reinterpret_cast<const float4*>(a.part_o + slot_of(p0 + u) * n + col));
   };
-  // per-head maximum and normaliser over all parts (np is small: a sequence of L tokens spans
-  // about L / (tokens per CTA) + 1 CTAs)
-  float* s_M = s_w + kCombineMaxParts * a.Hq;  // [Hq]
-  float* s_inv = s_M + a.Hq;                   // [Hq]
-  for (int h = threadIdx.x; h < a.Hq; h += kCombineThreads) {
-    float M = -INFINITY;
-    for (int p = 0; p < np; ++p) M = fmaxf(M, a.part_ml[(slot_of(p) * a.Hq + h) * 2]);
-    float L = 0.f;
-    for (int p = 0; p < np; ++p) {
-      const float2 ml = *reinterpret_cast<const float2*>(a.part_ml + (slot_of(p) * a.Hq + h) * 2);
-      L += exp2f(ml.x - M) * ml.y;
+  load(0);
+  auto stage = [&](int p0) {         // maxima and sums of the pieces p0 ..; a context of more than P pieces passes three times
+    __syncthreads();
+    for (int t = tid; t < min(P, np - p0) * a.Hq; t += kCombineThreads)
+      s_ml[t] = __ldcg(reinterpret_cast<const float2*>(a.part_ml + (slot_of(p0 + t / a.Hq) * a.Hq + t % a.Hq) * 2));
+    __syncthreads();
+  };
+  const bool once = np <= P;
+  for (int p0 = 0; p0 < np; p0 += P) {
+    stage(p0);
+    for (int h = tid; h < a.Hq; h += kCombineThreads) {
+      float M = p0 == 0 ? -INFINITY : s_M[h];
+      for (int p = 0; p < min(P, np - p0); ++p) M = fmaxf(M, s_ml[p * a.Hq + h].x);
+      s_M[h] = M;                    // its own head: no other thread reads it before the next barrier
     }
-    if (a.sink != nullptr) L += sink_term(a.sink[h], M);
-    s_M[h] = M;
-    s_inv[h] = a.bias != nullptr ? gate_of<__nv_bfloat16>(a, i, h) : 1.f / L;     // SIGM: M is 0
   }
-  __syncthreads();
-  constexpr int kVec = 4;
-  const int nvec = n / kVec;  // D is a multiple of 16 on this path
-  float4 acc[4];
-  // every thread owns up to 4 float4 columns (n <= 16 * 256 * 4 covers Hq*D <= 16384)
-  for (int base = 0; base < nvec; base += kCombineThreads * 4) {
-#pragma unroll
-    for (int u = 0; u < 4; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int p0 = 0; p0 < np; p0 += kCombineMaxParts) {
-      const int pc = min(kCombineMaxParts, np - p0);
-      __syncthreads();
-      for (int t = threadIdx.x; t < pc * a.Hq; t += kCombineThreads) {
-        const int p = p0 + t / a.Hq, h = t % a.Hq;
-        s_w[t] = exp2f(a.part_ml[(slot_of(p) * a.Hq + h) * 2] - s_M[h]) * s_inv[h];
+  for (int p0 = 0; p0 < np; p0 += P) {
+    if (!once) stage(p0);
+    for (int h = tid; h < a.Hq; h += kCombineThreads) {
+      const float M = s_M[h];
+      float L = p0 == 0 ? 0.f : s_inv[h];
+      for (int p = 0; p < min(P, np - p0); ++p) {
+        const float2 ml = s_ml[p * a.Hq + h];
+        L += exp2f(ml.x - M) * ml.y;
       }
-      __syncthreads();
+      if (p0 + P >= np) {
+        if (a.sink != nullptr) L += sink_term(a.sink[h], M);
+        L = a.bias != nullptr ? gate_of<__nv_bfloat16>(a, i, h) : 1.f / L;     // SIGM: M is 0
+      }
+      s_inv[h] = L;
+    }
+  }
+  const int head = in ? col / a.D : 0;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int p0 = 0; p0 < np; p0 += P) {
+    if (!once) stage(p0);
+    else __syncthreads();
+    const int pc = min(P, np - p0);
+    for (int t = tid; t < pc * a.Hq; t += kCombineThreads) s_w[t] = exp2f(s_ml[t].x - s_M[t % a.Hq]) * s_inv[t % a.Hq];
+    __syncthreads();
+    for (int q0 = 0; q0 < pc; q0 += kCombineAhead) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int vi = base + u * kCombineThreads + threadIdx.x;
-        if (vi < nvec) {
-          const int head = (vi * kVec) / a.D;
-          for (int p = 0; p < pc; ++p) {
-            const float4 x =
-                *reinterpret_cast<const float4*>(a.part_o + slot_of(p0 + p) * n + vi * kVec);
-            const float w = s_w[p * a.Hq + head];
-            acc[u].x += w * x.x;
-            acc[u].y += w * x.y;
-            acc[u].z += w * x.z;
-            acc[u].w += w * x.w;
-          }
+      for (int u = 0; u < kCombineAhead; ++u)
+        if (in && q0 + u < pc) {
+          const float w = s_w[(q0 + u) * a.Hq + head];
+          acc.x += w * x[u].x;
+          acc.y += w * x[u].y;
+          acc.z += w * x[u].z;
+          acc.w += w * x[u].w;
         }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int vi = base + u * kCombineThreads + threadIdx.x;
-      if (vi < nvec) {
-        uint2 packed;
-        packed.x = pack_bf16x2(acc[u].x, acc[u].y);
-        packed.y = pack_bf16x2(acc[u].z, acc[u].w);
-        *reinterpret_cast<uint2*>(op + vi * kVec) = packed;
-      }
+      load(p0 + q0 + kCombineAhead);
     }
   }
+  if (in) *reinterpret_cast<uint2*>(op) = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
 }
 
 // The combine follows the attention kernel in the stream and reads only what that kernel wrote: as a
 // programmatic dependent its launch and CTA placement overlap the attention kernel's tail.
 int launch_combine(const DecodeArgs& a, int batch, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(batch);
+  const int P = combine_parts(a.Hq);
+  cfg.gridDim = dim3(batch, (a.Hq * a.D / 4 + kCombineThreads - 1) / kCombineThreads);
   cfg.blockDim = dim3(kCombineThreads);
-  cfg.dynamicSmemBytes = (kCombineMaxParts + 2) * a.Hq * sizeof(float);
+  cfg.dynamicSmemBytes = (3 * P + 2) * a.Hq * sizeof(float);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, paged_decode_combine_kernel, a) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, paged_decode_combine_kernel, a, P) != cudaSuccess) {
     cudaGetLastError();
     return B200_ERR_LAUNCH;
   }
