@@ -8,7 +8,9 @@
 // the call is at position 0 starts from zero whatever its slot holds, so slots need no clearing when they
 // change hands.
 //
-// recurrence_step_kernel   one CTA per (sequence, head), tokens in order: decode, and sizes the scan does not take.
+// recurrence_step_kernel   one CTA per (sequence, head), tokens in order: decode, and sizes the other forms do not take.
+//
+// Prompts and portions in bf16 with heads of 64 or 128 run recurrence_chunk.cu, blocks of sixteen tokens on tensor cores.
 //
 // recurrence_scan_kernel   prompts and portions, cut into segments of seg_len tokens that run in parallel.  A segment
 //                          maps its entry state to D * S + P (D: product of its forget gates, P: its own writes), so

@@ -340,11 +340,31 @@ __global__ void __launch_bounds__(4 * D, D == 64 ? 2 : 1) recurrence_chunk_kerne
         mul(1, x[0], y[1]);
         mul(2, x[0], y[2]);
       }
+      bool odd = false;                            // a value that is not finite: it must not meet A's zeros of the tokens before it
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        uint32_t y[4];
-        ldmatrix_x4(y, smem_u32(&sm.a[st][i][r_in * ROWA + bh * 8]));
-        mul(i, vf, y);
+      for (int i = 0; i < 4; ++i) odd |= (vf[i] & 0x7f80u) == 0x7f80u || (vf[i] & 0x7f800000u) == 0x7f800000u;
+      if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int t = n * 8 + 2 * tq + (e & 1), col = vr + 8 * (e >> 1);
+            float sum = 0.f;
+#pragma unroll 1
+            for (int s = 0; s <= t; ++s) {
+              const int at = t * ROWA + s;
+              const float w = (__bfloat162float(sm.a[st][2][at]) + __bfloat162float(sm.a[st][1][at])) + __bfloat162float(sm.a[st][0][at]);
+              sum += w * __bfloat162float(sm.v[st][s * ROW + col]);
+            }
+            O[0][n][e] += sum;
+          }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          uint32_t y[4];
+          ldmatrix_x4(y, smem_u32(&sm.a[st][i][r_in * ROWA + bh * 8]));
+          mul(i, vf, y);
+        }
       }
 #pragma unroll
       for (int n = 0; n < 2; ++n)

@@ -264,6 +264,25 @@ def test_gated_recurrence_blocks_of_sixteen_tokens(H, d, lens):
     assert (got[free] == 7.0).all()
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("at", [0, 21, 31, 32])
+def test_gated_recurrence_value_that_is_not_finite_reaches_no_earlier_token(d, at):
+    from llm_from_scratch_b200 import ops
+    H, n, w = 2, 40, 2 * d
+    g = gen(at)
+    x = torch.randn(2 * n, 3 * w, generator=g).bfloat16()
+    y = x.clone()
+    y[at, 2 * w + 3] = float("inf")
+    args = [t.cuda() for t in (torch.randn(w, generator=g), torch.rand(w, generator=g), torch.ones(d))]
+    cu = torch.tensor([0, n, 2 * n], dtype=torch.int32).cuda()
+    run = lambda p: ops.gated_recurrence(*p.cuda().split(w, 1), *args, 1e-5, torch.zeros(2, H, d, d).cuda(),
+                                         torch.arange(2).cuda(), cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=n)
+    a, b = run(x), run(y)
+    assert torch.equal(a[n:], b[n:]) and torch.isfinite(a.float()).all()
+    if at:                   # summed in another order: a bf16 step (2^-7 of the value) here and there
+        assert rel(b[:at], a[:at].cpu()) <= 2.0 ** -7
+
+
 def test_store_kv_rows_of_unequal_widths():
     from llm_from_scratch_b200 import ops
     for wk, wv, dtype in ((64, 96, torch.bfloat16), (21, 10, torch.bfloat16), (12, 20, torch.float32), (3, 5, torch.float32)):
