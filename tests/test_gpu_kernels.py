@@ -812,6 +812,19 @@ def test_moe_grouped_gemm_matches_per_expert_matmuls(counts, k, n, swiglu):
     assert torch.equal(again, ops.moe_grouped_gemm(x, w, offs, bias, swiglu=swiglu))
 
 
+@pytest.mark.parametrize("counts,k,n", [([256, 257, 384, 385, 128, 1, 0, 640], 128, 264),                          # weights stay in L2: short tiles last
+                                        ([300, 1, 257, 0, 700, 128, 129, 256, 90, 385, 511, 40, 65], 2048, 1024)])   # 109 MB of them: in order
+def test_moe_grouped_gemm_row_tiles_of_one_and_two_halves(counts, k, n):
+    ops = _ops()
+    offs = torch.tensor(np.cumsum(counts), dtype=torch.int32, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.randn(sum(counts), k, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(len(counts), 2 * n, k, generator=g, device="cuda") * k ** -0.5).bfloat16()
+    got, want = ops.moe_grouped_gemm(x, w, offs, None, swiglu=True), _grouped_reference(x, w, offs, None, True)
+    ops.check_status()
+    assert ((got.float() - want.float()).abs() <= 2e-2 * want.float().abs() + 2e-2).all()
+
+
 @pytest.mark.parametrize("swiglu,big", [(True, False), (False, False), (True, True), (False, True)])
 def test_moe_grouped_gemm_dense_tail_is_one_more_weight_set(swiglu, big):
     """Rows after the grouped ones that all use weight set E (a shared expert in the same launch), in
