@@ -6,6 +6,7 @@ the current CUDA stream.  Nothing here computes on the CPU; a CPU tensor is an e
 from __future__ import annotations
 
 import array
+import functools
 import math
 from dataclasses import dataclass
 
@@ -34,16 +35,20 @@ def _dt(t: torch.Tensor) -> int:
 
 
 def _cuda(*ts: torch.Tensor | None) -> torch.device:
-    dev = None
+    # device numbers instead of device objects: a call checks five to ten tensors, and building an object for each
+    # took longer than the rest of its checks
+    first, dev = None, -1
     for t in ts:
         if t is None:
             continue
-        if not t.is_cuda:
+        i = t.get_device()
+        if i < 0 or not t.is_cuda:
             raise ValueError("b200 ops take CUDA tensors only (there is no CPU path)")
-        if dev is not None and t.device != dev:
+        if first is None:
+            first, dev = t, i
+        elif i != dev:
             raise ValueError("all tensors must be on the same device")
-        dev = t.device
-    return dev
+    return None if first is None else first.device
 
 
 def _stream() -> int:
@@ -152,6 +157,11 @@ def store_rows(rows: torch.Tensor, cache: torch.Tensor, slot_mapping: torch.Tens
                                  status_word(dev).data_ptr(), _stream()), "store_rows")
 
 
+@functools.lru_cache(maxsize=256)
+def _decode_workspace_bytes(B: int, Hq: int, Hkv: int, D: int, dtype: int) -> int:
+    return lib.b200_paged_decode_gqa_workspace_bytes(B, Hq, Hkv, D, dtype)
+
+
 def paged_decode_gqa(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                      block_tables: torch.Tensor, context_lens: torch.Tensor, scale: float,
                      out: torch.Tensor | None = None, sink: torch.Tensor | None = None) -> torch.Tensor:
@@ -180,8 +190,7 @@ def paged_decode_gqa(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
         out = torch.empty((B, Hq, Dv), dtype=q.dtype, device=q.device)
     elif out.shape != (B, Hq, Dv) or out.dtype != q.dtype or not out.is_contiguous():
         raise ValueError("out must be a contiguous [B, Hq, Dv] tensor of q's dtype")
-    need = lib.b200_paged_decode_gqa_workspace_bytes(B, Hq, Hkv, D, _dt(q))
-    ws = workspace(dev, need, "decode")
+    ws = workspace(dev, _decode_workspace_bytes(B, Hq, Hkv, D, _dt(q)), "decode")
     if sink is not None or Dv != D:
         check(lib.b200_paged_decode_sink(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
                                          block_tables.data_ptr(), block_tables.stride(0), context_lens.data_ptr(), B, Hq,
