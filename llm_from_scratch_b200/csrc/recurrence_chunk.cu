@@ -20,13 +20,16 @@
 // a warp).  Both halves in one warp, with two barriers per block, took 549 us where this takes 227 (8 prompts of 1,024 tokens
 // x 16 heads x 128 x 128); the scalar walk, 5 FMA per state element and token over two passes, took 786.
 //
-// Against 64 bits the states are 3.6e-8 .. 1.4e-7 off, the scalar walk's 3.5e-8 .. 1.4e-7.
+// Against 64 bits the states are 3.6e-8 .. 1.4e-7 off, the scalar walk's 3.5e-8 .. 1.4e-7.  Long memories (1,024 to 32,768 tokens,
+// values of one sign): channels that keep 0.999 per token 1.6e-7 .. 2.4e-7, the walk's 4e-6 .. 1e-5; 0.9999 1.9e-7 .. 4.8e-7, the
+// walk's 5e-6 .. 9e-5.  With the state as the accumulator of K~^T V and plain products of gates it was 1.35e-5 and 1.6e-4 (224 us).
 #include "recurrence_common.cuh"
 
 namespace b200 {
 namespace {
 
 constexpr int BT = 16;                         // tokens per block
+constexpr int kOwn = 4;                        // accumulators of K~^T V in flight
 
 // x (two values) -> three packed bf16 pairs whose sum is x to 24 bits
 __device__ __forceinline__ void split3(f32x2 x, uint32_t& h, uint32_t& m, uint32_t& l) {
@@ -41,6 +44,9 @@ __device__ __forceinline__ void split3(f32x2 x, uint32_t& h, uint32_t& m, uint32
   l = pack_bf16x2(y.x, y.y);
 }
 __device__ __forceinline__ void split3(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) { split3(pack2(x0, x1), h, m, l); }
+
+// 1 - (1 - a)(1 - b)
+__device__ __forceinline__ float both(float a, float b) { return fmaf(-a, b, a + b); }
 
 template <int D>
 struct __align__(16) ChunkSmem {
@@ -105,7 +111,7 @@ __global__ void __launch_bounds__(4 * D, D == 64 ? 2 : 1) recurrence_chunk_kerne
       }
       cp_async_commit();
     };
-    float dec0 = 1.f, dec1 = 1.f;                    // product of the segment's gates, lanes of the last four tokens
+    float dec = 1.f, owed = 0.f;                     // of channel c + (tq & 1): product of the segment's gates; see below
     auto gate_block = [&](int b) {
       float f[4][2], k[4][2], q[4][2];
       const int sw = c ^ (tq * 8);
@@ -124,7 +130,7 @@ __global__ void __launch_bounds__(4 * D, D == 64 ? 2 : 1) recurrence_chunk_kerne
           *reinterpret_cast<float2*>(sm.qf + at) = make_float2(q[i][0], q[i][1]);
         }
       }
-      float before[2], behind[2], all[2];            // products of the other threads' tokens
+      float before[2], behind[2], all[2], loss[2];   // products of the other threads' tokens and of all; 1 - product of the own
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const float own = (f[0][j] * f[1][j]) * (f[2][j] * f[3][j]);
@@ -134,7 +140,6 @@ __global__ void __launch_bounds__(4 * D, D == 64 ? 2 : 1) recurrence_chunk_kerne
         if (tq >= 2) up *= y;
         y = __shfl_up_sync(0xffffffffu, up, 1, 4);
         before[j] = tq >= 1 ? y : 1.f;
-        all[j] = up;
         float dn = own;
         y = __shfl_down_sync(0xffffffffu, dn, 1, 4);
         if (tq <= 2) dn *= y;
@@ -142,11 +147,8 @@ __global__ void __launch_bounds__(4 * D, D == 64 ? 2 : 1) recurrence_chunk_kerne
         if (tq <= 1) dn *= y;
         y = __shfl_down_sync(0xffffffffu, dn, 1, 4);
         behind[j] = tq <= 2 ? y : 1.f;
-      }
-      if (tq == 3) {
-        *reinterpret_cast<float2*>(sm.gamma[b & 1] + c) = make_float2(all[0], all[1]);
-        dec0 *= all[0];
-        dec1 *= all[1];
+        all[j] = tq == 3 ? up : dn * before[j];
+        loss[j] = both(both(k[0][j], k[1][j]), both(k[2][j], k[3][j]));
       }
       auto put = [&](__nv_bfloat16 (&dst)[3][BT * ROW], int t, float x0, float x1) {
         uint32_t h, m, l;
@@ -166,6 +168,21 @@ __global__ void __launch_bounds__(4 * D, D == 64 ? 2 : 1) recurrence_chunk_kerne
         put(sm.k[b & 1], tq * 4 + i, k[i][0] * behind[0], k[i][1] * behind[1]);
         behind[0] *= f[i][0];
         behind[1] *= f[i][1];
+      }
+      // F_15.  Gates just below one round to a product that is always too small, (1 - e)(1 - e') losing an e e' of less than half
+      // a step: block after block that would be a decay of its own.  There F_15 is 1 - loss, loss from the write gates 1 - f, and
+      // makes up for what the rounding of the block before took (`owed`, relative; 2 - F stands for 1 / F near one).
+      {
+        const bool odd = tq & 1;
+        const float y = __shfl_xor_sync(0xffffffffu, odd ? loss[0] : loss[1], 1), two = both(odd ? loss[1] : loss[0], y);
+        const float gone = both(two, __shfl_xor_sync(0xffffffffu, two, 2));
+        float gamma = odd ? all[1] : all[0];
+        const bool near_one = fabsf(gone) < 0.25f;
+        const float x = 1.f - gone, more = fmaf(x, owed, 1.f - x - gone);
+        gamma = near_one ? x + more : gamma;
+        owed = near_one ? (x - gamma + more) * (2.f - gamma) : 0.f;
+        if (LOCAL) dec *= gamma;
+        if (tq >= 2) sm.gamma[b & 1][c + odd] = gamma;
       }
     };
 
@@ -270,10 +287,7 @@ __global__ void __launch_bounds__(4 * D, D == 64 ? 2 : 1) recurrence_chunk_kerne
       }
       __syncthreads();
     }
-    if (LOCAL && tq == 3) {
-      float* dec = sc.seg_decay + (static_cast<int64_t>(number) * a.H + head) * D;
-      *reinterpret_cast<float2*>(dec + c) = make_float2(dec0, dec1);
-    }
+    if (LOCAL && tq >= 2) sc.seg_decay[(static_cast<int64_t>(number) * a.H + head) * D + c + (tq & 1)] = dec;
     return;
   }
 
@@ -372,23 +386,32 @@ __global__ void __launch_bounds__(4 * D, D == 64 ? 2 : 1) recurrence_chunk_kerne
         for (int e = 0; e < 4; ++e)
           sm.o[(n * 8 + 2 * tq + (e & 1)) * LDO + vr + 8 * (e >> 1)] = (O[2][n][e] + O[1][n][e]) + O[0][n][e];
     }
+    // S^T <- diag(gamma) S^T + (K~^T V)^T, the product in accumulators of its own: a tensor core cuts the low bits of the sums it adds
+    // to, always to one side, and a state that keeps 0.999 of itself per token would carry the cuts of a thousand tokens
 #pragma unroll
-    for (int n = 0; n < NK; ++n) {
-      const float2 gm = *reinterpret_cast<const float2*>(sm.gamma[st] + n * 8 + 2 * tq);
-      const f32x2 x = pack2(gm.x, gm.y);
-      const float2 u = unpack2(mul2(pack2(S[n][0], S[n][1]), x)), w = unpack2(mul2(pack2(S[n][2], S[n][3]), x));
-      S[n][0] = u.x, S[n][1] = u.y, S[n][2] = w.x, S[n][3] = w.y;
-    }
+    for (int n0 = 0; n0 < NK; n0 += kOwn) {
+      float P[kOwn][4];
 #pragma unroll
-    for (int i = 2; i >= 0; --i)
+      for (int n = 0; n < kOwn; ++n) P[n][0] = P[n][1] = P[n][2] = P[n][3] = 0.f;
 #pragma unroll
-      for (int n = 0; n < NK; n += 2) {
-        uint32_t y[4];
-        ldmatrix_x4_trans(y, smem_u32(&sm.k[st][i][t_in * ROW + (n + th) * 8]));
-        const uint32_t y0[2] = {y[0], y[1]}, y1[2] = {y[2], y[3]};
-        mma_bf16_16816(S[n], vf, y0);
-        mma_bf16_16816(S[n + 1], vf, y1);
+      for (int i = 2; i >= 0; --i)
+#pragma unroll
+        for (int n = 0; n < kOwn; n += 2) {
+          uint32_t y[4];
+          ldmatrix_x4_trans(y, smem_u32(&sm.k[st][i][t_in * ROW + (n0 + n + th) * 8]));
+          const uint32_t y0[2] = {y[0], y[1]}, y1[2] = {y[2], y[3]};
+          mma_bf16_16816(P[n], vf, y0);
+          mma_bf16_16816(P[n + 1], vf, y1);
+        }
+#pragma unroll
+      for (int n = 0; n < kOwn; ++n) {
+        float (&x)[4] = S[n0 + n];
+        const f32x2 f = *reinterpret_cast<const f32x2*>(sm.gamma[st] + (n0 + n) * 8 + 2 * tq);
+        const float2 u = unpack2(fma2(pack2(x[0], x[1]), f, pack2(P[n][0], P[n][1])));
+        const float2 w = unpack2(fma2(pack2(x[2], x[3]), f, pack2(P[n][2], P[n][3])));
+        x[0] = u.x, x[1] = u.y, x[2] = w.x, x[3] = w.y;
       }
+    }
   };
 
   __syncthreads();

@@ -264,6 +264,36 @@ def test_gated_recurrence_blocks_of_sixteen_tokens(H, d, lens):
     assert (got[free] == 7.0).all()
 
 
+@pytest.mark.parametrize("d,H,n,seqs", [(64, 2, 8192, 1), (128, 16, 8192, 10), (128, 1, 32768, 1), (64, 16, 32768, 10)])
+@pytest.mark.parametrize("bias", [6.9, 9.2])
+def test_gated_recurrence_of_long_memories_is_as_exact_as_the_walk(d, H, n, seqs, bias):
+    """Channels that keep 0.999 or 0.9999 of themselves per token and still write, values of one sign, so that nothing averages out.
+    State against 64 bits, beside the walk's (the same call with gate constants off a 16-byte boundary).  Bound: a block's
+    factor is within a rounding of its product and makes up for the last one, so what grows is one rounding of the state per block
+    of sixteen tokens over a memory of 1 / (1 - f) tokens, and a write gate carries 3e-7: 1e-6 in all."""
+    from llm_from_scratch_b200 import ops
+    w, g = H * d, torch.Generator(device="cuda").manual_seed(n + d)
+    x = torch.randn(n * seqs, 3 * w, device="cuda", generator=g, dtype=torch.bfloat16)
+    x[:, w:2 * w] *= 0.3
+    x[:, 2 * w:] += 1
+    consts = torch.full((w + 1,), bias, device="cuda"), torch.zeros(w, device="cuda"), torch.ones(d, device="cuda")
+    cu = torch.arange(0, (seqs + 1) * n, n, dtype=torch.int32, device="cuda")
+    z = x[:n, w:w + d].double() + consts[0][0].double()                     # first head of the first sequence
+    f, k, v = torch.sigmoid(z), torch.sigmoid(-z), x[:n, 2 * w:2 * w + d].double()
+    want = torch.zeros(d, d, device="cuda", dtype=torch.float64)
+    for t in range(0, n, 64):
+        F = f[t:t + 64].log().cumsum(0)
+        want = F[-1].exp()[:, None] * want + (k[t:t + 64] * (F[-1:] - F).exp()).T @ v[t:t + 64]
+    off = []
+    for fb in (consts[0][:w], consts[0][1:]):
+        state = torch.zeros(seqs, H, d, d, device="cuda")
+        ops.gated_recurrence(x[:, :w], x[:, w:2 * w], x[:, 2 * w:], fb, *consts[1:], 1e-5, state, torch.arange(seqs, device="cuda"),
+                             cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=n)
+        off.append(((state[0, 0].double() - want).norm() / want.norm()).item())
+    ops.check_status()
+    assert off[0] <= min(off[1], 1e-6), off
+
+
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("at", [0, 21, 31, 32])
 def test_gated_recurrence_value_that_is_not_finite_reaches_no_earlier_token(d, at):
