@@ -165,10 +165,11 @@ __global__ void __launch_bounds__(kThreads) decode_cluster_kernel(const ClusterA
       float p[4];
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const float mn = fmaxf(m[nt][e], mx[e]), al = fast_exp2(m[nt][e] - mn);
+        const float mn = fmaxf(m[nt][e], mx[e]), ref = mn == -INFINITY ? 0.f : mn;     // scores of -inf alone: weights 0
+        const float al = fast_exp2(m[nt][e] - ref);
         m[nt][e] = mn;
-        p[e] = fast_exp2(x[e] - mn);
-        p[e + 2] = fast_exp2(x[e + 2] - mn);
+        p[e] = fast_exp2(x[e] - ref);
+        p[e + 2] = fast_exp2(x[e + 2] - ref);
         l[nt][e] = l[nt][e] * al + p[e] + p[e + 2];
 #pragma unroll
         for (int mt = 0; mt < KS; ++mt) {

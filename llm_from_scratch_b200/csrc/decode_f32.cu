@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kThreads, 3) decode_f32_kernel(const DecodeF32
       float p[OWN];
 #pragma unroll
       for (int c = 0; c < OWN; ++c) {
-        p[c] = in[c] ? fast_exp2(x[c] - m_own[c]) : 0.f;
+        p[c] = x[c] == -INFINITY ? 0.f : fast_exp2(x[c] - m_own[c]);       // a maximum of -inf must not meet another
         l_own[c] += p[c];
       }
       // ---- outputs

@@ -179,6 +179,26 @@ def test_decode_in_clusters_and_in_one_stream(Hq, Hkv, D, bs, lens, sink):
         assert_close(got, want, torch.bfloat16)
 
 
+@pytest.mark.parametrize("dtype,D", [(torch.bfloat16, 128), (torch.float32, 32), (torch.float32, 64), (torch.float32, 128)])
+@pytest.mark.parametrize("gone", [(16, 32), (0, 16), (0, 8), (64, 128), (100, 164), (1, 300), (0, 299)])
+def test_decode_of_keys_whose_scores_are_minus_infinity(dtype, D, gone):
+    """They weigh nothing, also where a block, a trip of a lane, a warp or a whole CTA of a cluster holds no others."""
+    ops, orc = _ops(), _oracle()
+    case, q, kc, vc = _decode_case([300], 8, 2, D, 16, dtype, seed=D)
+    q[..., 0] = 1
+    rows = torch.from_numpy(case.block_tables[0, :19]).long()[:, None] * 16 + torch.arange(16)
+    rows = rows.flatten()[:300]
+    left = torch.tensor([i for i in range(300) if not gone[0] <= i < gone[1]])
+    k, v = kc.flatten(0, 1)[rows[left]], vc.flatten(0, 1)[rows[left]]
+    kc.view(-1, 2, D)[rows[gone[0]:gone[1]], :, 0] = float("-inf")
+    p = torch.softmax(torch.einsum("hd,nhd->hn", q[0].double(), k.double().repeat_interleave(4, 1)) * D ** -0.5, -1)
+    want = torch.einsum("hn,nhd->hd", p, v.double().repeat_interleave(4, 1))[None]
+    got = ops.paged_decode_gqa(q.cuda(), kc.cuda(), vc.cuda(), torch.from_numpy(case.block_tables).cuda(),
+                               torch.from_numpy(case.context_lens).cuda(), D ** -0.5)
+    ops.check_status()
+    assert_close(got, want, dtype)
+
+
 def test_paged_decode_bf16_single_short_sequence_and_stale_table_entries():
     # entries past ceil(len/16) hold stale ids outside the pool: they must never be read
     case, q, kc, vc = _decode_case([20], 32, 8, 128, 16, torch.bfloat16, seed=3)
