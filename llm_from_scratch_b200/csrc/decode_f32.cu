@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kThreads, 3) decode_f32_kernel(const DecodeF32
       sum += f * *cluster.map_shared_rank(&c_l[g], r);
     }
     if (a.sink != nullptr && M > -INFINITY) sum += exp2f(a.sink[head0 + g] * 1.4426950408889634f - M);
-    a.out[(static_cast<int64_t>(seq) * a.Hq + head0 + g) * D + d] = sum > 0.f ? x / sum : 0.f;
+    a.out[(static_cast<int64_t>(seq) * a.Hq + head0 + g) * D + d] = sum == 0.f ? 0.f : x / sum;   // 0: no key; a NaN stays one
   }
   cluster.sync();            // nobody leaves while another CTA reads its shared memory
 }

@@ -719,6 +719,7 @@ __global__ void __launch_bounds__(kSimpleWarps * 32) paged_decode_simple_kernel(
       continue;
     }
     dot *= a.scale_log2;
+    if (dot == -INFINITY) continue;           // weighs nothing, and must not meet a maximum of -inf
     const float mn = fmaxf(m, dot);
     const float al = exp2f(m - mn), pw = exp2f(dot - mn);
     l = l * al + pw;
@@ -757,7 +758,7 @@ __global__ void __launch_bounds__(kSimpleWarps * 32) paged_decode_simple_kernel(
   for (int d = threadIdx.x; d < Dv; d += blockDim.x) {
     float v = 0.f;
     for (int w = 0; w < kSimpleWarps; ++w) v += wgt[w] * s_acc[w][d];
-    op[d] = from_float<T>(Lsum > 0.f ? v / Lsum : 0.f);
+    op[d] = from_float<T>(Lsum == 0.f ? 0.f : v / Lsum);     // 0: no key; a NaN stays one
   }
 }
 

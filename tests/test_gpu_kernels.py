@@ -179,7 +179,7 @@ def test_decode_in_clusters_and_in_one_stream(Hq, Hkv, D, bs, lens, sink):
         assert_close(got, want, torch.bfloat16)
 
 
-@pytest.mark.parametrize("dtype,D", [(torch.bfloat16, 128), (torch.float32, 32), (torch.float32, 64), (torch.float32, 128)])
+@pytest.mark.parametrize("dtype,D", [(torch.bfloat16, 128), (torch.float32, 32), (torch.float32, 64), (torch.float32, 80), (torch.float32, 128)])
 @pytest.mark.parametrize("gone", [(16, 32), (0, 16), (0, 8), (64, 128), (100, 164), (1, 300), (0, 299)])
 def test_decode_of_keys_whose_scores_are_minus_infinity(dtype, D, gone):
     """They weigh nothing, also where a block, a trip of a lane, a warp or a whole CTA of a cluster holds no others."""
@@ -197,6 +197,18 @@ def test_decode_of_keys_whose_scores_are_minus_infinity(dtype, D, gone):
                                torch.from_numpy(case.context_lens).cuda(), D ** -0.5)
     ops.check_status()
     assert_close(got, want, dtype)
+
+
+@pytest.mark.parametrize("dtype,D,page", [(torch.float32, 32, 16), (torch.float32, 64, 16), (torch.float32, 128, 16), (torch.float32, 80, 16),
+                                          (torch.bfloat16, 128, 16), (torch.bfloat16, 64, 16), (torch.bfloat16, 64, 5)])
+@pytest.mark.parametrize("n,at", [(300, 0), (300, 170), (1, 0)])
+def test_a_broken_key_row_is_seen_in_the_output(dtype, D, page, n, at):
+    """A NaN in one visible key makes the rows of its query heads NaN, not zeros, and no others."""
+    ops = _ops()
+    case, q, kc, vc = _decode_case([n], 8, 2, D, page, dtype, seed=D)
+    kc[case.block_tables[0, at // page], at % page, 1, 3] = float("nan")
+    got = _run_decode(case, q, kc, vc, D ** -0.5)
+    assert torch.isfinite(got[0, :4]).all() and torch.isnan(got[0, 4:]).all()
 
 
 def test_paged_decode_bf16_single_short_sequence_and_stale_table_entries():
