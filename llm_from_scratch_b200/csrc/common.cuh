@@ -153,6 +153,12 @@ inline int launch_result() {
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? B200_OK : B200_ERR_LAUNCH;
 }
+// Of cudaLaunchKernelEx: a failure also stays behind as the runtime's last error, which the next launch would take for its own.
+inline int launch_result(cudaError_t e) {
+  if (e == cudaSuccess) return launch_result();
+  cudaGetLastError();
+  return B200_ERR_LAUNCH;
+}
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Cached per-device SM count (read-only after first use).

@@ -284,11 +284,7 @@ int launch(const ClusterArgs& a, int batch, int ranks, cudaStream_t s) {
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, decode_cluster_kernel<NT>, a) != cudaSuccess) {
-    cudaGetLastError();
-    return B200_ERR_LAUNCH;
-  }
-  return launch_result();
+  return launch_result(cudaLaunchKernelEx(&cfg, decode_cluster_kernel<NT>, a));
 }
 
 }  // namespace

@@ -313,11 +313,7 @@ int launch_heads(const DecodeF32Args& a, int batch, int ranks, cudaStream_t s) {
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, decode_f32_kernel<D, GC>, a) != cudaSuccess) {
-    cudaGetLastError();
-    return B200_ERR_LAUNCH;
-  }
-  return launch_result();
+  return launch_result(cudaLaunchKernelEx(&cfg, decode_f32_kernel<D, GC>, a));
 }
 
 template <int D>

@@ -476,11 +476,7 @@ int launch(const GemmArgs& a, const CUtensorMap& tw, const CUtensorMap& tx, dim3
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = early ? 1 : 0;
-  if (cudaLaunchKernelEx(&cfg, moe_gemm_kernel<NPASS, STAGES>, a, tw, tx) != cudaSuccess) {
-    cudaGetLastError();
-    return B200_ERR_LAUNCH;
-  }
-  return launch_result();
+  return launch_result(cudaLaunchKernelEx(&cfg, moe_gemm_kernel<NPASS, STAGES>, a, tw, tx));
 }
 
 }  // namespace
@@ -614,10 +610,6 @@ extern "C" int b200_lm_head_argmax(const void* hidden, const void* w, const void
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, lm_head_argmax_finish_kernel, static_cast<const unsigned long long*>(a.amax_key),
-                         tiles, static_cast<int>(num_rows), tokens) != cudaSuccess) {
-    cudaGetLastError();
-    return B200_ERR_LAUNCH;
-  }
-  return launch_result();
+  return launch_result(cudaLaunchKernelEx(&cfg, lm_head_argmax_finish_kernel, static_cast<const unsigned long long*>(a.amax_key),
+                                          tiles, static_cast<int>(num_rows), tokens));
 }

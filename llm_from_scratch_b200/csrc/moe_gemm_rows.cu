@@ -403,7 +403,7 @@ int moe_gemm_rows_launch(const void* x, const void* w, const void* bias, void* o
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = early ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, moe_gemm_rows_kernel, a, tx, tw) == cudaSuccess ? launch_result() : B200_ERR_LAUNCH;
+  return launch_result(cudaLaunchKernelEx(&cfg, moe_gemm_rows_kernel, a, tx, tw));
 }
 
 }  // namespace b200

@@ -632,11 +632,7 @@ int launch_combine(const DecodeArgs& a, int batch, cudaStream_t s) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, paged_decode_combine_kernel, a, P) != cudaSuccess) {
-    cudaGetLastError();
-    return B200_ERR_LAUNCH;
-  }
-  return launch_result();
+  return launch_result(cudaLaunchKernelEx(&cfg, paged_decode_combine_kernel, a, P));
 }
 
 }  // namespace

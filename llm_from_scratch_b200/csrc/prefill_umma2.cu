@@ -590,7 +590,7 @@ int launch2(const Args2& a, const CUtensorMap& tq, const CUtensorMap& tk, const 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = a.beside_store ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, a, tq, tk, tkt, tv) == cudaSuccess ? launch_result() : B200_ERR_LAUNCH;
+  return launch_result(cudaLaunchKernelEx(&cfg, kern, a, tq, tk, tkt, tv));
 }
 
 }  // namespace

@@ -447,7 +447,7 @@ int prefill_umma4_launch(const void* q, const void* k, const void* v, void* out,
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = a.beside_store ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, prefill_umma4_kernel, a, tq, tk, tv) == cudaSuccess ? launch_result() : B200_ERR_LAUNCH;
+  return launch_result(cudaLaunchKernelEx(&cfg, prefill_umma4_kernel, a, tq, tk, tv));
 }
 
 }  // namespace b200

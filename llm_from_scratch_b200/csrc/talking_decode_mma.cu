@@ -421,7 +421,7 @@ int launch_decode_as(const TalkArgs& a, const DecodeParts& parts, size_t smem, c
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, talking_merge_kernel, a, parts) == cudaSuccess ? launch_result() : B200_ERR_LAUNCH;
+  return launch_result(cudaLaunchKernelEx(&cfg, talking_merge_kernel, a, parts));
 }
 
 template <int HP, int NT, int MAXU>
