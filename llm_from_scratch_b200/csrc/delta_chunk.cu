@@ -260,6 +260,15 @@ __device__ __forceinline__ void copy_piece(uint8_t* dst, const void* src, uint32
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src),
                "r"(bytes), "r"(bar) : "memory");
 }
+// For every thread of the CTA, each with whether its wait for the copies counted on `bar` ended: true if all did.  If not, the CTA
+// is about to leave, and copies that were only late must have landed before it gives its shared memory back (waited for with a limit).
+__device__ __forceinline__ bool all_landed(bool here, bool pending, uint32_t bar, uint32_t parity) {
+  if (!__syncthreads_or(!here)) return true;
+  int never = 0;
+  if (pending) umma::mbar_wait(bar, parity, &never, 1 << 16);
+  __syncthreads();
+  return false;
+}
 // The rows of a chunk's nt tokens, `width` columns each; zeros behind them up to `padded` columns and C rows.
 __device__ __forceinline__ void copy_rows(uint8_t* dst, int pitch, const __nv_bfloat16* src, int64_t stride, int nt, int width,
                                           int padded, int tid, int threads, uint32_t bar) {
@@ -349,13 +358,14 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const ChunkArgs args
   const int r_in = (lane & 7) + (lane >> 4) * 8, bh = (lane >> 3) & 1;      // B operand, rows = n: (n lo, k lo) (n lo, k hi) (n hi, ...)
   const int t_in = (lane & 7) + ((lane >> 3) & 1) * 8, th = lane >> 4;      // B operand transposed, rows = k
   for (int j = 0; j < chunks; ++j) {
-    if (!umma::mbar_wait(bar_of(j), (j >> 1) & 1, &s_abort)) {
+    const bool here = umma::mbar_wait(bar_of(j), (j >> 1) & 1, &s_abort);
+    if (!here) {
       s_abort = 1;
       report(a.status, B200_ERR_TIMEOUT);
     }
     umma::fence_async_proxy();                         // outputs were staged where the next copies go
-    __syncthreads();                                   // chunk j has landed; everyone has left the other stage
-    if (s_abort) return;
+    // chunk j, the only one on its way, has landed; everyone has left the other stage
+    if (!all_landed(here, true, bar_of(j), (j >> 1) & 1)) return;
     if (j + 1 < chunks) fetch(j + 1);
     uint8_t* stp = smem + (j & 1) * lay.bytes;
     const uint32_t st = sbase + (j & 1) * lay.bytes;
@@ -601,18 +611,19 @@ __global__ void __launch_bounds__(256, 1) delta_split_kernel(const ChunkArgs arg
   // byte offset of eight columns of a row
   auto at_row = [&](int r, int c8) { return r * 128 + ((c8 ^ (r & 7)) << 4); };
   auto bar_of = [&](int j) { return smem_u32(&s_bars[outputs][j & 1]); };
-  // chunk j of this half has landed, `rows` bytes of rows at `tile`, for every thread: false if it never will
+  // chunk j of this half, the only one on its way, has landed, `rows` bytes of rows at `tile`, for every thread of both halves: false
+  // if one of them never will
   auto landed = [&](int j, bool wait, uint8_t* tile, int rows) {
-    if (wait && !umma::mbar_wait(bar_of(j), (j >> 1) & 1, &s_abort)) {
+    const bool here = !wait || umma::mbar_wait(bar_of(j), (j >> 1) & 1, &s_abort);
+    if (!here) {
       s_abort = 1;
       report(a.status, B200_ERR_TIMEOUT);
     }
     const int nt = info.len - j * C;
-    if (wait && nt < C)
+    if (wait && here && nt < C)
       for (int i = tid; i < rows / 16; i += NT)
         if ((i / 8) % C >= nt) reinterpret_cast<uint4*>(tile)[i] = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
-    return s_abort == 0;
+    return all_landed(here, wait, bar_of(j), (j >> 1) & 1);
   };
   auto blob_of = [&](int j) { return blob0 + static_cast<size_t>(j) * a.H * kBlobBytes; };
   // this lane's words of a state (0) or U (1) of chunk j
