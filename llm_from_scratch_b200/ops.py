@@ -158,7 +158,9 @@ def store_rows(rows: torch.Tensor, cache: torch.Tensor, slot_mapping: torch.Tens
 
 
 @functools.lru_cache(maxsize=256)
-def _decode_workspace_bytes(B: int, Hq: int, Hkv: int, D: int, dtype: int) -> int:
+def _decode_workspace_bytes(current_device: int, B: int, Hq: int, Hkv: int, D: int, dtype: int) -> int:
+    """The size follows the current device's number of SMs; without one the library answers for 148, which is not kept."""
+    check(min(lib.b200_sm_count(), 0), "paged_decode_gqa")
     return lib.b200_paged_decode_gqa_workspace_bytes(B, Hq, Hkv, D, dtype)
 
 
@@ -190,7 +192,7 @@ def paged_decode_gqa(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
         out = torch.empty((B, Hq, Dv), dtype=q.dtype, device=q.device)
     elif out.shape != (B, Hq, Dv) or out.dtype != q.dtype or not out.is_contiguous():
         raise ValueError("out must be a contiguous [B, Hq, Dv] tensor of q's dtype")
-    ws = workspace(dev, _decode_workspace_bytes(B, Hq, Hkv, D, _dt(q)), "decode")
+    ws = workspace(dev, _decode_workspace_bytes(torch._C._cuda_getDevice(), B, Hq, Hkv, D, _dt(q)), "decode")
     if sink is not None or Dv != D:
         check(lib.b200_paged_decode_sink(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
                                          block_tables.data_ptr(), block_tables.stride(0), context_lens.data_ptr(), B, Hq,

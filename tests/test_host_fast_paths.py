@@ -234,3 +234,37 @@ def test_decode_window_planning_respects_length_and_pool_limits():
         sched.block_manager.open_block(a)
     a.num_tokens = 8                                     # next lengths 9.. would start a block
     assert sched.plan_decode_window(seqs, 4, 300) == 1
+
+
+def test_scratch_size_of_a_decode_shape_is_kept_per_device(monkeypatch):
+    """Devices with other numbers of SMs get their own answers, and one without an answer gets none that stays."""
+    from llm_from_scratch_b200 import _lib, ops
+
+    class Library:
+        sms = 148
+
+        def b200_sm_count(self):
+            return self.sms
+
+        def b200_paged_decode_gqa_workspace_bytes(self, *shape):
+            return (self.sms if self.sms > 0 else 148) * 1000
+
+        def b200_strerror(self, code):
+            return b"no device"
+
+    fake = Library()
+    monkeypatch.setattr(ops, "lib", fake)
+    monkeypatch.setattr(_lib, "lib", fake)
+    shape = (3, 16, 4, 64, 1)
+    ops._decode_workspace_bytes.cache_clear()
+    try:
+        assert ops._decode_workspace_bytes(0, *shape) == 148000
+        fake.sms = 132
+        assert ops._decode_workspace_bytes(0, *shape) == 148000 and ops._decode_workspace_bytes(1, *shape) == 132000
+        fake.sms = -7
+        with pytest.raises(_lib.B200Error):
+            ops._decode_workspace_bytes(2, *shape)
+        fake.sms = 160
+        assert ops._decode_workspace_bytes(2, *shape) == 160000
+    finally:
+        ops._decode_workspace_bytes.cache_clear()
