@@ -79,8 +79,10 @@ __global__ void __launch_bounds__(kThreads) decode_cluster_kernel(const ClusterA
     len64 = cap;
   }
   const int len = len64 > 0 ? static_cast<int>(len64) : 0;
-  // ---- this CTA's blocks, of them every kWarps-th for a warp
-  const int blocks = (len + kTok - 1) / kTok, per = (blocks + ranks - 1) / ranks;
+  // ---- this CTA's blocks, of them every kWarps-th for a warp.  The first `used` CTAs share the context, a block per warp at least;
+  // the others leave: a barrier of the cluster counts the threads that are still there, and nobody reads what they hold.
+  const int blocks = (len + kTok - 1) / kTok, per = max((blocks + ranks - 1) / ranks, kWarps), used = max((blocks + per - 1) / per, 1);
+  if (rank >= used) return;
   const int lo = min(rank * per, blocks) + warp, hi = min((rank + 1) * per, blocks);
   const int mine = lo < hi ? (hi - lo + kWarps - 1) / kWarps : 0;
   const int32_t* table = a.bt + static_cast<int64_t>(seq) * a.bt_stride;
@@ -231,16 +233,16 @@ __global__ void __launch_bounds__(kThreads) decode_cluster_kernel(const ClusterA
     *reinterpret_cast<float4*>(&c_o[head][d]) = x;
     if (d == 0) c_m[head] = M, c_l[head] = sum;
   }
-  if (ranks > 1) cluster.sync();
+  if (used > 1) cluster.sync();
   else __syncthreads();
   // ---- CTAs of the cluster: every one finishes its share of the columns
-  for (int i = rank * kThreads + tid; i < G * (D / 2); i += ranks * kThreads) {
+  for (int i = rank * kThreads + tid; i < G * (D / 2); i += used * kThreads) {
     const int head = i / (D / 2), d = i % (D / 2) * 2;
     float mr[8], lr[8], M = -INFINITY;
     float2 y[8];
 #pragma unroll
     for (int r = 0; r < 8; ++r)
-      if (r < ranks) {
+      if (r < used) {
         mr[r] = *cluster.map_shared_rank(&c_m[head], r);
         lr[r] = *cluster.map_shared_rank(&c_l[head], r);
         y[r] = *reinterpret_cast<const float2*>(cluster.map_shared_rank(&c_o[head][d], r));
@@ -249,7 +251,7 @@ __global__ void __launch_bounds__(kThreads) decode_cluster_kernel(const ClusterA
     float sum = 0.f, x0 = 0.f, x1 = 0.f;
 #pragma unroll
     for (int r = 0; r < 8; ++r)
-      if (r < ranks) {
+      if (r < used) {
         const float f = mr[r] == -INFINITY ? 0.f : exp2f(mr[r] - M);
         sum += f * lr[r];
         x0 += f * y[r].x;
@@ -259,7 +261,7 @@ __global__ void __launch_bounds__(kThreads) decode_cluster_kernel(const ClusterA
     const float inv = sum > 0.f ? 1.f / sum : 0.f;     // an empty context gives zeros
     *reinterpret_cast<uint32_t*>(a.out + (static_cast<int64_t>(seq) * a.Hq + h * G + head) * D + d) = pack_bf16x2(x0 * inv, x1 * inv);
   }
-  if (ranks > 1) cluster.sync();                       // nobody leaves while another CTA reads its shared memory
+  if (used > 1) cluster.sync();                        // nobody leaves while another CTA reads its shared memory
 }
 
 template <int NT>
@@ -299,16 +301,18 @@ int decode_cluster_launch(const void* q, const void* kc, const void* vc, void* o
   if (D != kDim || sms <= 0 || batch > 65535) return B200_ERR_UNSUPPORTED;
   const int64_t pairs = static_cast<int64_t>(batch) * Hkv, keys = bt_stride * sub * kTok, wave = 2 * static_cast<int64_t>(sms);
   // CTAs per context: one wave of them, none with less than a block per warp; where a context may leave a CTA more than 1,024
-  // tokens up to four waves, which evens out unequal contexts (32 x 128 .. 8,192 tokens at 32/8 heads: 51 against 72 us)
+  // tokens up to two waves, which evens out unequal contexts (16 of 128 .. 8,192 tokens: four CTAs 36 us, two 48, one 76; with
+  // four waves 32 short contexts under a wide table took longer than in one stream: 256 tokens 18 against 14 us).
   int ranks = 1;
-  while (ranks < 8 && static_cast<int64_t>(ranks) * kWarps * kTok < keys && pairs * ranks * 2 <= wave * (keys / ranks > 1024 ? 4 : 1))
+  while (ranks < 8 && static_cast<int64_t>(ranks) * kWarps * kTok < keys && pairs * ranks * 2 <= wave * (keys / ranks > 1024 ? 2 : 1))
     ranks *= 2;
-  // The streaming form keeps two corners: contexts of up to 256 tokens in more than two waves of clusters, where a CTA's fixed
-  // cost shows (256 x 64 tokens: 30 against 23 us), and contexts that may leave a CTA more than 4,096 tokens, where the longest
-  // sets the time (128 x 128 .. 8,192 tokens: 173 against 166 us).  Elsewhere (32/8 heads) one of 700 tokens takes 5 against 17 us,
-  // 64 x 64 .. 1,024 33 against 39, 256 x 700 118 against 124.
-  if (keys <= 256 && pairs * ranks > 2 * wave) return B200_ERR_UNSUPPORTED;
-  if (keys / ranks > 4096) return B200_ERR_UNSUPPORTED;
+  // Only the width of the table is known here, so the line lies where no contexts that fit it are slower than in one stream by more
+  // than the stream's own scatter.  Times in us, clusters / stream, 32/8 heads; `64+n`: one context of n tokens among those of 64.
+  //   one context of 700 tokens 5.5 / 16, of 8,192 13 / 70; 16 of 64 4.1 / 7.8, of 2,000 23 / 37
+  //   32 (256 pairs): of 64 4.6 / 8.0, of 700 12.4 / 24; under a table of 8,192 (two CTAs each) of 128 .. 8,192 72 / 70
+  //   64 (512 pairs): of 64 7.6 / 9.0, of 64 .. 1,024 21 / 24, but 64+4000 41 / 25
+  //   128 (1,024 pairs): of 64 13.5 / 9.2, of 700 62 / 65; 512: of 16 41 / 14, of 700 215 / 228
+  if (keys > (pairs * 2 <= wave ? 32768 : pairs <= wave ? 8192 : pairs <= 2 * wave ? 2048 : 0)) return B200_ERR_UNSUPPORTED;
   const ClusterArgs a{static_cast<const __nv_bfloat16*>(q), static_cast<const uint8_t*>(kc), static_cast<const uint8_t*>(vc),
                       static_cast<__nv_bfloat16*>(out), bt, bt_stride, lens, Hq, Hkv, sub, num_blocks, scale_log2, sink, status};
   return Hq / Hkv > 8 ? launch<2>(a, batch, ranks, s) : launch<1>(a, batch, ranks, s);

@@ -88,6 +88,8 @@ __global__ void __launch_bounds__(kThreads, 3) decode_f32_kernel(const DecodeF32
   // ---- the CTA's range of the context
   constexpr int TRIP = kWarps * TW * kUnroll;
   const int per = ((len + ranks - 1) / ranks + TRIP - 1) / TRIP * TRIP;
+  const int used = per > 0 ? (len + per - 1) / per : 1;       // CTAs with keys; a barrier of the cluster does not count those that left
+  if (rank >= used) return;
   const int lo = min(rank * per, len), hi = min(lo + per, len);
   const int shift = (a.bs & (a.bs - 1)) == 0 ? __ffs(a.bs) - 1 : -1;
   auto page_of = [&](int t) { return shift >= 0 ? t >> shift : t / a.bs; };
@@ -272,14 +274,15 @@ __global__ void __launch_bounds__(kThreads, 3) decode_f32_kernel(const DecodeF32
     c_o[g][d] = x;
     if (d == 0) c_m[g] = M, c_l[g] = sum;
   }
-  cluster.sync();
+  if (used > 1) cluster.sync();
+  else __syncthreads();
   // every CTA finishes its share of the columns
-  for (int i = rank * kThreads + tid; i < GC * D; i += ranks * kThreads) {
+  for (int i = rank * kThreads + tid; i < GC * D; i += used * kThreads) {
     const int g = i / D, d = i % D;
     float M = -INFINITY;
-    for (int r = 0; r < ranks; ++r) M = fmaxf(M, *cluster.map_shared_rank(&c_m[g], r));
+    for (int r = 0; r < used; ++r) M = fmaxf(M, *cluster.map_shared_rank(&c_m[g], r));
     float x = 0.f, sum = 0.f;
-    for (int r = 0; r < ranks; ++r) {
+    for (int r = 0; r < used; ++r) {
       const float mr = *cluster.map_shared_rank(&c_m[g], r);
       const float f = mr == -INFINITY ? 0.f : exp2f(mr - M);
       x += f * *cluster.map_shared_rank(&c_o[g][d], r);
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(kThreads, 3) decode_f32_kernel(const DecodeF32
     if (a.sink != nullptr && M > -INFINITY) sum += exp2f(a.sink[head0 + g] * 1.4426950408889634f - M);
     a.out[(static_cast<int64_t>(seq) * a.Hq + head0 + g) * D + d] = sum == 0.f ? 0.f : x / sum;   // 0: no key; a NaN stays one
   }
-  cluster.sync();            // nobody leaves while another CTA reads its shared memory
+  if (used > 1) cluster.sync();            // nobody leaves while another CTA reads its shared memory
 }
 
 template <int D, int GC>
