@@ -294,18 +294,36 @@ int launch_rows(const PrefillF32Args& a, int max_seqlen_q, int64_t total_q, cuda
   if (sms <= 0) sms = 148;
   // tiles of 64 rows move fewer operands per product, tiles of 32 give a small batch more CTAs: the line is where the former
   // still give every SM two (4 prompts of 100 tokens at 16/4 x 64: 18.6 us in tiles of 64, 16.5 us in tiles of 32; 8 prompts
-  // of 500 tokens at 16/4 x 32: 79 and 99 us)
-  if (total_q * a.Hq / 64 >= 2 * sms) return launch_tiles<D, 4>(a, max_seqlen_q, s);
+  // of 500 tokens at 16/4 x 32: 79 and 99 us).  Sequences of up to 32 rows fill no more than the smaller tile (256 x 8 tokens behind 64 at
+  // 16/16 x 128: 532 us in tiles of 64, 304 in tiles of 32).
+  if (static_cast<int64_t>(max_seqlen_q) * (a.Hq / a.Hkv) > 32 && total_q * a.Hq / 64 >= 2 * sms) return launch_tiles<D, 4>(a, max_seqlen_q, s);
   return launch_tiles<D, 2>(a, max_seqlen_q, s);
+}
+
+// Whether the general kernel, a warp per row that reads every key, is the faster one: short portions leave most of a 32-row tile
+// empty, and a tile of keys costs a CTA as much for one key as for all.  Times of both in us from what they measured at 16/4 x 64, 32/8 x
+// 128, 16/16 x 32, 16/16 x 128 and 8/1 x 128, 1 to 256 sequences of 1 to 16 tokens behind 0 to 1,024: a chain of keys or tiles where
+// the batch is small, the rate of all warps or CTAs where it is large.  64 x 1 token at 16/4 x 64: 3.2 us, in tiles 10.6; 256 x 1 behind 64 at
+// 16/16 x 128: 172 and 302; 256 x 1 behind 64 at 16/4 x 64: 100 and 61.
+bool general_is_faster(const PrefillF32Args& a, int D, int64_t total_q, int max_seqlen_q, int max_seqlen_k) {
+  const int64_t rows = static_cast<int64_t>(max_seqlen_q) * (a.Hq / a.Hkv);
+  if (rows > 32 || max_seqlen_k > 128) return false;
+  const double rate = max_seqlen_q == 1 ? 1600 : max_seqlen_q <= 3 ? 2100 : 3100;                   // rows x keys a us
+  const double all = static_cast<double>(total_q) * a.Hq * (max_seqlen_k - max_seqlen_q / 2) / rate;
+  const double chain = 0.75 * max_seqlen_k, general = 2.5 + (all > chain ? all : chain);
+  const int tiles = (max_seqlen_k + tile_keys(D) - 1) / tile_keys(D);
+  const double tile_all = static_cast<double>(a.num_seqs) * a.Hkv * (tiles + 0.5) / (D == 128 ? 41 : D == 64 ? 38 : 75);
+  const double tile_chain = 3 + (D == 32 ? 4.2 : 7.5) * tiles;
+  return general < 0.9 * (tile_all > tile_chain ? tile_all : tile_chain);
 }
 
 }  // namespace
 
-// B200_ERR_UNSUPPORTED: a shape, stride or alignment that the tiles do not take (the general kernel does)
+// B200_ERR_UNSUPPORTED: a shape, stride or alignment that the tiles do not take, or sizes at which the general kernel is the faster one
 int prefill_f32_launch(const void* q, const void* k, const void* v, void* out, int64_t q_stride, int64_t k_stride,
                        int64_t v_stride, int64_t total_q, const int32_t* cu_q, const int32_t* cu_k, int num_seqs,
-                       int max_seqlen_q, int Hq, int Hkv, int Dqk, int Dv, float scale, const void* kc, const void* vc,
-                       const int32_t* bt, int64_t bt_stride, int bs, int64_t num_blocks, const float* sink, int32_t* status,
+                       int max_seqlen_q, int max_seqlen_k, int Hq, int Hkv, int Dqk, int Dv, float scale, const void* kc,
+                       const void* vc, const int32_t* bt, int64_t bt_stride, int bs, int64_t num_blocks, const float* sink, int32_t* status,
                        cudaStream_t s) {
   if (Dqk != Dv || (Dqk != 32 && Dqk != 64 && Dqk != 128) || static_cast<int64_t>(num_seqs) * Hkv > 2147483647LL) return B200_ERR_UNSUPPORTED;
   const void* kp = bt ? kc : k;
@@ -316,6 +334,7 @@ int prefill_f32_launch(const void* q, const void* k, const void* v, void* out, i
   PrefillF32Args a{static_cast<const float*>(q), static_cast<const float*>(kp), static_cast<const float*>(vp),
                    static_cast<float*>(out), q_stride, k_stride, v_stride, cu_q, cu_k, num_seqs, Hq, Hkv,
                    scale * 1.4426950408889634f, bt, bt_stride, bs, num_blocks, sink, status};
+  if (general_is_faster(a, Dqk, total_q, max_seqlen_q, max_seqlen_k)) return B200_ERR_UNSUPPORTED;
   if (Dqk == 32) return launch_rows<32>(a, max_seqlen_q, total_q, s);
   if (Dqk == 64) return launch_rows<64>(a, max_seqlen_q, total_q, s);
   return launch_rows<128>(a, max_seqlen_q, total_q, s);

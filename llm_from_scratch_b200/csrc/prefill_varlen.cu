@@ -189,8 +189,8 @@ int prefill_umma_launch(const void* q, const void* k, const void* v, void* out, 
 // fp32 at head sizes 32 / 64 / 128 (prefill_f32.cu)
 int prefill_f32_launch(const void* q, const void* k, const void* v, void* out, int64_t q_stride, int64_t k_stride,
                        int64_t v_stride, int64_t total_q, const int32_t* cu_q, const int32_t* cu_k, int num_seqs,
-                       int max_seqlen_q, int Hq, int Hkv, int Dqk, int Dv, float scale, const void* kc, const void* vc,
-                       const int32_t* bt, int64_t bt_stride, int bs, int64_t num_blocks, const float* sink, int32_t* status,
+                       int max_seqlen_q, int max_seqlen_k, int Hq, int Hkv, int Dqk, int Dv, float scale, const void* kc,
+                       const void* vc, const int32_t* bt, int64_t bt_stride, int bs, int64_t num_blocks, const float* sink, int32_t* status,
                        cudaStream_t s);
 
 }  // namespace b200
@@ -305,7 +305,7 @@ static int prefill_attention(const void* q, const void* k, const void* v, void* 
     if (rc != B200_ERR_UNSUPPORTED) return rc;
   } else {
     const int rc = prefill_f32_launch(q, k, v, out, q_token_stride, k_token_stride, v_token_stride, total_q_tokens,
-                                      cu_seqlens_q, cu_seqlens_k, num_seqs, max_seqlen_q, num_q_heads, num_kv_heads,
+                                      cu_seqlens_q, cu_seqlens_k, num_seqs, max_seqlen_q, max_seqlen_k, num_q_heads, num_kv_heads,
                                       head_dim_qk, head_dim_v, scale, k_cache, v_cache, block_tables, bt_stride, block_size,
                                       num_blocks, sink, status, s);
     if (rc != B200_ERR_UNSUPPORTED) return rc;

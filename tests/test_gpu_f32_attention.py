@@ -65,6 +65,21 @@ def test_paged_prefix_and_blocks_outside_the_pool(page, Hq, Hkv, D):
     assert ops.read_status_code() != 0
 
 
+@pytest.mark.parametrize("Hq,Hkv,D", [(16, 4, 64), (16, 16, 128), (16, 16, 32)])
+@pytest.mark.parametrize("n", [1, 70])
+@pytest.mark.parametrize("q_len,prefix", [(1, 0), (1, 30), (2, 127), (3, 62), (8, 0), (8, 24), (9, 0)])
+def test_short_portions(Hq, Hkv, D, n, q_len, prefix):
+    """Sizes on both sides of the line between tiles and a warp per row; the other side is always the warp per row."""
+    from llm_from_scratch_b200 import ops
+    k_len = q_len + prefix
+    case = deal_blocks([k_len] * n, 16, np.random.default_rng(n), pad_blocks=1)
+    kc, vc = _randn(3, case.num_blocks, 16, Hkv, D), _randn(4, case.num_blocks, 16, Hkv, D)
+    tables, q = torch.from_numpy(case.block_tables).cuda(), _randn(5, n * q_len, Hq, D)
+    args = (q, None, None, _cu([q_len] * n), _cu([k_len] * n), q_len, k_len, D ** -0.5, kc, vc, tables)
+    _same(ops.prefill_varlen(*args), ops.prefill_varlen(*args, out=_off_boundary(q.shape)))
+    ops.check_status()
+
+
 def test_values_a_row_does_not_see_stay_out_of_it():
     from llm_from_scratch_b200 import ops
     lens, Hq, Hkv, D = [100, 90], 8, 2, 64
