@@ -297,7 +297,10 @@ struct ScanLayout {
   }
 };
 
-template <int DK>
+// ROWS: rows come as bulk copies, else as 16-byte pieces by all threads.  A bulk copy per row is issued by one thread after the other, on
+// the warps of the chain, which few warps feel more than they gain: 16 sequences of 1,024 tokens, heads of 128 x 128 589 us in rows and
+// 601 in pieces, 128 x 64 312 and 290, 32 x 64 262 and 234, 16 x 16 532 and 458; T, P and the factors, one copy, are a gain at every size.
+template <int DK, bool ROWS>
 __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const ChunkArgs args) {
   using Lay = ScanLayout<DK>;
   constexpr int ROWK = Lay::ROWK, NK = DK / 8;
@@ -330,16 +333,26 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const ChunkArgs args
     const int nt = min(C, info.len - j * C);
     const int64_t tok = info.tok0 + j * C;
     if (tid == 0) {
-      umma::mbar_expect_tx(bar_of(j), nt * (2 * dk + dv) * 2 + kBlobBytes);
+      umma::mbar_expect_tx(bar_of(j), (ROWS ? nt * (2 * dk + dv) * 2 : 0) + kBlobBytes);
       copy_piece(st + lay.p, blob0 + static_cast<size_t>(j) * a.H * kBlobBytes, kBlobBytes, bar_of(j));      // T, P, factors
     }
     auto rows = [&](int at, int pitch, const void* src, int off, int width, int padded) {
-      copy_rows(st + at, pitch, static_cast<const __nv_bfloat16*>(src) + tok * a.act_stride + off, a.act_stride, nt, width, padded, tid,
-                NT, bar_of(j));
+      const __nv_bfloat16* from = static_cast<const __nv_bfloat16*>(src) + tok * a.act_stride + off;
+      if constexpr (ROWS) {
+        copy_rows(st + at, pitch, from, a.act_stride, nt, width, padded, tid, NT, bar_of(j));
+      } else {
+        const int pieces = padded / 8;
+        for (int i = tid; i < C * pieces; i += NT) {
+          const int r = i / pieces, c = i - r * pieces;
+          const bool ok = r < nt && c * 8 < width;
+          cp_async16(smem_u32(st + at + r * pitch + c * 16), from + (ok ? r * a.act_stride + c * 8 : 0), ok ? 16 : 0);
+        }
+      }
     };
     rows(lay.k, ROWK * 2, a.k, kh * dk, dk, DK);
     rows(lay.q, ROWK * 2, a.q, kh * dk, dk, DK);
     rows(lay.v, lay.rowv * 2, a.v, head * dv, dv, dv);
+    if constexpr (!ROWS) cp_async_commit();
   };
 
   // S^T: rows 16 warp + g (+ 8), columns 8 n + 2 tq (+ 1)
@@ -363,6 +376,7 @@ __global__ void __launch_bounds__(256, 1) delta_scan_kernel(const ChunkArgs args
       s_abort = 1;
       report(a.status, B200_ERR_TIMEOUT);
     }
+    if constexpr (!ROWS) cp_async_wait<0>();
     umma::fence_async_proxy();                         // outputs were staged where the next copies go
     // chunk j, the only one on its way, has landed; everyone has left the other stage
     if (!all_landed(here, true, bar_of(j), (j >> 1) & 1)) return;
@@ -913,10 +927,11 @@ int launch(const ChunkArgs& c, int64_t total_tokens, cudaStream_t s) {
   const size_t prep = sizeof(PrepSmem<DK>);
   const ScanLayout<DK> lay(c.d.dv);
   const size_t scan = 2 * static_cast<size_t>(lay.bytes);
+  constexpr int kRowsFrom = DK == 128 ? 96 : 1 << 30;      // value columns from which rows come as bulk copies
+  auto walk = DK == 128 && c.d.dv >= kRowsFrom ? delta_scan_kernel<DK, DK == 128> : delta_scan_kernel<DK, false>;
   if (cudaFuncSetAttribute(delta_prepare_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(prep)) !=
           cudaSuccess ||
-      cudaFuncSetAttribute(delta_scan_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(scan)) !=
-          cudaSuccess)
+      cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(scan)) != cudaSuccess)
     return B200_ERR_LAUNCH;
   delta_prepare_kernel<DK><<<dim3(static_cast<unsigned>(chunk_count(c.d.n, total_tokens)), c.d.H), kPrepThreads, prep, s>>>(c);
   CUtensorMap tq, tk, tv;
@@ -927,7 +942,7 @@ int launch(const ChunkArgs& c, int64_t total_tokens, cudaStream_t s) {
       return B200_ERR_LAUNCH;
     delta_split_kernel<<<dim3(c.d.H, c.d.n), c.d.dv * 4, SplitLayout::bytes, s>>>(c, tq, tk, tv);
   } else {
-    delta_scan_kernel<DK><<<dim3(c.d.H, c.d.n), c.d.dv * 2, scan, s>>>(c);
+    walk<<<dim3(c.d.H, c.d.n), c.d.dv * 2, scan, s>>>(c);
   }
   return launch_result();
 }
