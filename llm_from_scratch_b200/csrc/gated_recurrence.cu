@@ -482,7 +482,8 @@ extern "C" int b200_gated_recurrence(const void* q, const void* f, const void* v
                aligned16(f) && aligned16(v);
     // bf16 and heads of 64 or 128 run on tensor cores: 8 x 1,024 tokens x 16 heads of 128 227 us against 786 us
     const bool chunks = dtype == B200_DTYPE_BF16 && recurrence_chunk_shape(dim_k, dim_v) && sc.async && aligned16(f_bias) &&
-                        aligned16(lower) && aligned16(norm_w) && aligned16(out);
+                        aligned16(lower) && aligned16(norm_w) && aligned16(out) &&
+                        (max_seqlen_q > sc.seg_len || recurrence_chunk_pays(num_seqs, total_tokens, max_seqlen_q, num_heads, dim_k));
     // never shorter than the scan's: the workspace is sized for those
     if (chunks) sc.seg_len = max(sc.seg_len, recurrence_chunk_seg_len(total_tokens, max_seqlen_q, num_heads));
     const int64_t segments = total_tokens / sc.seg_len + num_seqs;

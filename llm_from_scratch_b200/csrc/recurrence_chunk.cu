@@ -450,6 +450,17 @@ int launch(const RecArgs& a, const ScanArgs& sc, int64_t segments, bool chained,
 
 }  // namespace
 
+// For sequences that the scan would not cut.  A block costs the same for one token as for sixteen.  In one wave of CTAs the longest
+// sequence sets the time (16 x 16 heads of 64: 3 tokens 7.7 us, token by token 6.5; 6 tokens 7.8 and 9.2); above that the rates of both
+// count, in ns per sequence and block or token from 1 to 256 sequences of 2 to 33 tokens (256 x 16 heads of 64: 5 tokens 99 us, token by
+// token 68; 16 tokens 104 and 120; of 128: 5 tokens 240 and 190, 16 tokens 247 and 338).
+bool recurrence_chunk_pays(int n, int64_t total_tokens, int max_seqlen_q, int H, int D) {
+  const int sms = sm_count_cached();
+  if (static_cast<int64_t>(n) * H <= (D == 64 ? 2 : 1) * static_cast<int64_t>(sms > 0 ? sms : 148)) return max_seqlen_q >= 5;
+  const double tokens = static_cast<double>(total_tokens) / n, blocks = max_seqlen_q <= BT ? 1 : static_cast<int64_t>((tokens + BT - 1) / BT);
+  return D == 64 ? 12.9 + 10.5 * blocks < 9.5 + 1.23 * tokens : 35.3 + 22.3 * blocks < 29.5 + 3.3 * tokens;
+}
+
 int recurrence_chunk_seg_len(int64_t total_tokens, int max_seqlen_q, int H) {
   // one CTA per SM and head; whole sequences as long as the longest takes less than two such shares, since cutting costs
   // two more launches, half of the work again and three passes over the states

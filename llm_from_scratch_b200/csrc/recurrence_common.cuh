@@ -43,6 +43,7 @@ struct ScanArgs {
 
 // prompts and portions on tensor cores (recurrence_chunk.cu): bf16, dk = dv = 64 or 128, 16-byte aligned rows
 inline bool recurrence_chunk_shape(int dk, int dv) { return dk == dv && (dk == 64 || dk == 128); }
+bool recurrence_chunk_pays(int n, int64_t total_tokens, int max_seqlen_q, int H, int D);
 int recurrence_chunk_seg_len(int64_t total_tokens, int max_seqlen_q, int H);
 int recurrence_chunk_launch(const RecArgs& a, const ScanArgs& sc, int64_t segments, bool chained, cudaStream_t s);
 

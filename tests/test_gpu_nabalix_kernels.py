@@ -230,7 +230,7 @@ def test_gated_recurrence_in_portions_and_steps(H, dk, dv, dtype, tol):
 
 
 @pytest.mark.parametrize("H,d", [(3, 64), (2, 128), (16, 64), (9, 128)])
-@pytest.mark.parametrize("lens", [[700, 1, 16, 17], [32, 15, 1, 31, 2], [129, 128, 127]])
+@pytest.mark.parametrize("lens", [[700, 1, 16, 17], [32, 15, 1, 31, 2], [129, 128, 127], [4, 1], [5, 1], [12, 8] * 10, [2] * 20, [17] * 20])
 def test_gated_recurrence_blocks_of_sixteen_tokens(H, d, lens):
     """Whole and cut sequences around the edges of a block and of a segment, some of them continued; channels that forget
     everything within a token or nothing at all.  State: what a token wrote is multiplied by one fp32 gate per later token, each
