@@ -31,9 +31,10 @@ constexpr int kStepThreads = 256;
 // Threads are RG row groups x CL column units of V columns; a unit walks the key channels rg, rg + RG, ...  The first kAhead state
 // rows of a unit are requested before the gates are formed: one decoded token is a chain of latencies (64 sequences x 8 heads x
 // 64 x 64: 8.4 us, 10.5 with the rows behind the gates; 128 x 16 x 128 x 128: 55 and 78).
-constexpr int kAhead = 8;
-template <typename T, int V>
-__global__ void __launch_bounds__(kStepThreads) recurrence_step_kernel(const RecArgs a, int CL) {
+// With eight of them in registers fewer CTAs fit an SM, so units with fewer rows have a form with one or four (256 x 16 x 32 x 32:
+// 28 us, in the form with eight 38).
+template <typename T, int V, int kAhead>
+__global__ void __launch_bounds__(kStepThreads, V == 4 && kAhead == 1 ? 6 : 3) recurrence_step_kernel(const RecArgs a, int CL) {
   extern __shared__ float sm[];
   const int dk = a.dk, dv = a.dv, head = blockIdx.x;
   float* sf = sm;              // [dk] forget gate
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(kStepThreads) recurrence_step_kernel(const Rec
     const T* fp = static_cast<const T*>(a.f) + row + head * dk;
     const T* vp = static_cast<const T*>(a.v) + row + head * dv;
     const bool zero = info.fresh && t == 0;
-    float4 ahead[V == 4 ? kAhead : 1];
+    float4 ahead[kAhead];
     auto request = [&](int c, int r0) {           // rows r0, r0 + RG, ... of unit c
 #pragma unroll
       for (int j = 0; j < (V == 4 ? kAhead : 0); ++j) {
@@ -141,7 +142,9 @@ int launch_step(const RecArgs& a, int n, bool vec, cudaStream_t s) {
   int CL = 8;
   while (CL < units && CL < kStepThreads) CL *= 2;
   const size_t smem = (3 * static_cast<size_t>(a.dk) + a.dv + kStepThreads * V + 8) * sizeof(float);
-  auto kern = vec ? recurrence_step_kernel<T, 4> : recurrence_step_kernel<T, 1>;
+  const int rows = (a.dk * CL + kStepThreads - 1) / kStepThreads;        // of a unit
+  auto kern = !vec ? recurrence_step_kernel<T, 1, 1> : rows <= 1 ? recurrence_step_kernel<T, 4, 1>
+                   : rows <= 4 ? recurrence_step_kernel<T, 4, 4> : recurrence_step_kernel<T, 4, 8>;
   if (smem > 40 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                static_cast<int>(smem)) != cudaSuccess)
     return B200_ERR_LAUNCH;
