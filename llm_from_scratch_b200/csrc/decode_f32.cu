@@ -324,10 +324,14 @@ int launch_dim(const DecodeF32Args& a, int batch, cudaStream_t s) {
   int sms = sm_count_cached();
   if (sms <= 0) sms = 148;
   const int G = a.Hq / a.Hkv, GC = G % 4 == 0 ? 4 : G % 2 == 0 ? 2 : 1;
-  // CTAs per context: as many as still run in one wave of four per SM, none with less than a trip of its own; where contexts
-  // may be long, up to two waves, which evens out batches of unequal contexts (128 sequences, log-uniform from 32 to 2048
-  // tokens: 41 against 49 us; but 64 sequences of up to 1024 tokens: 28 against 26 us)
+  // CTAs per context: doubled up to four an SM, none with less than a trip of its own; where contexts may be long, up to eight an SM,
+  // which evens out batches of unequal contexts.  Three CTAs fit an SM at head sizes 32 and 64, two at 128, so four are more than one
+  // round; the line is where the times lie, not a wave (one, two, four, eight CTAs per context, 64 .. 1,024 tokens: 64 sequences at 16/4 x
+  // 64 19.5, 17.0, 19.2, 25.8 us, 32 at 32/8 x 128 34, 32, 38, 52; 128 .. 8,192 tokens, 64 at 16/4 x 64 129, 75, 64, 65).
   const int64_t pairs = static_cast<int64_t>(batch) * (a.Hq / GC), keys = a.bt_stride * a.bs;
+  // The general kernel keeps contexts of up to eight tokens, where the merges are the call (one token at 16/4 x 64: 4.7 against 2.8 us), and
+  // large batches of up to sixteen where no heads share the rows (256 x 16 at 16/16 x 32: 28 against 19).
+  if (keys <= 8 || (keys <= 16 && GC == 1 && pairs >= 2048)) return B200_ERR_UNSUPPORTED;
   const int trip = kWarps * (32 / (D / 8)) * kUnroll;
   int ranks = 1;
   while (ranks < 8 && static_cast<int64_t>(ranks) * trip < keys &&
@@ -340,7 +344,7 @@ int launch_dim(const DecodeF32Args& a, int batch, cudaStream_t s) {
 
 }  // namespace
 
-// B200_ERR_UNSUPPORTED: a shape or alignment that the general kernel takes
+// B200_ERR_UNSUPPORTED: a shape or alignment that the general kernel takes, or contexts too short for clusters
 int decode_f32_launch(const void* q, const void* kc, const void* vc, void* out, const int32_t* bt, int64_t bt_stride,
                       const int64_t* lens, int batch, int Hq, int Hkv, int D, int Dv, int bs, int64_t num_blocks,
                       float scale_log2, const float* sink, int32_t* status, cudaStream_t s) {

@@ -96,7 +96,8 @@ def test_values_a_row_does_not_see_stay_out_of_it():
 @pytest.mark.parametrize("page", [1, 16, 48])
 @pytest.mark.parametrize("Hq,Hkv,D,lens", [
     (16, 4, 64, [700]), (4, 4, 32, [1, 0, 7, 8, 9, 300]), (6, 2, 128, [33, 500, 16]), (32, 8, 128, [100, 900] * 8),
-    (16, 4, 64, [2, 0, *range(1, 130, 2)]), (8, 1, 64, [63, 64, 65] * 40), (3, 1, 32, [400] * 300)])
+    (16, 4, 64, [2, 0, *range(1, 130, 2)]), (8, 1, 64, [63, 64, 65] * 40), (3, 1, 32, [400] * 300), (16, 16, 32, [16, 3, 9] * 50),
+    (16, 4, 64, [8, 1, 5])])
 def test_decode(page, Hq, Hkv, D, lens):
     from llm_from_scratch_b200 import ops
     case = deal_blocks(lens, page, np.random.default_rng(1), pad_blocks=2)
