@@ -192,18 +192,20 @@ def paged_decode_gqa(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
         out = torch.empty((B, Hq, Dv), dtype=q.dtype, device=q.device)
     elif out.shape != (B, Hq, Dv) or out.dtype != q.dtype or not out.is_contiguous():
         raise ValueError("out must be a contiguous [B, Hq, Dv] tensor of q's dtype")
-    ws = workspace(dev, _decode_workspace_bytes(torch._C._cuda_getDevice(), B, Hq, Hkv, D, _dt(q)), "decode")
+    current = torch._C._cuda_getDevice()
+    ws = workspace(dev, _decode_workspace_bytes(current, B, Hq, Hkv, D, _dt(q)), "decode")
+    stream = torch._C._cuda_getCurrentRawStream(current)
     if sink is not None or Dv != D:
         check(lib.b200_paged_decode_sink(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
                                          block_tables.data_ptr(), block_tables.stride(0), context_lens.data_ptr(), B, Hq,
                                          Hkv, D, Dv, bs, nb, float(scale), _ptr(sink), ws.data_ptr(), ws.numel(), _dt(q),
-                                         status_word(dev).data_ptr(), _stream()), "paged_decode_sink")
+                                         status_word(dev).data_ptr(), stream), "paged_decode_sink")
         return out
     check(lib.b200_paged_decode_gqa(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
                                     out.data_ptr(), block_tables.data_ptr(),
                                     block_tables.stride(0), context_lens.data_ptr(), B, Hq, Hkv, D,
                                     bs, nb, float(scale), ws.data_ptr(), ws.numel(), _dt(q),
-                                    status_word(dev).data_ptr(), _stream()), "paged_decode_gqa")
+                                    status_word(dev).data_ptr(), stream), "paged_decode_gqa")
     return out
 
 
