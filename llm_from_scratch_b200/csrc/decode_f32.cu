@@ -8,9 +8,9 @@
 // A lane copies its own pieces of the rows a trip ahead into a ring of its own; the block numbers of a CTA's range are
 // read into shared memory first, because a table read per trip, even one trip ahead, set the pace.
 //
-// Measured at 64 sequences of 64 to 1024 tokens, 16/4 heads x 64: 26 us (the general kernel, a CTA per sequence and query
-// head: 306 us); 128 sequences of 2048 tokens, 32/8 x 128: 343 us, 6.3 TB/s.  With the table read inside the trips and a full
-// reduction of every score the two took 32 and 457 us.
+// Measured at 64 sequences of 64 to 1024 tokens, 16/4 heads x 64: 28 us (the general kernel, a CTA per sequence and query
+// head: 307 us); 128 sequences of 2048 tokens, 32/8 x 128: 346 us, 6.2 TB/s.  With the table read inside the trips and a full
+// reduction of every score the latter took 457 us.
 #include <cooperative_groups.h>
 
 #include "sequences.cuh"

@@ -29,10 +29,9 @@ namespace {
 constexpr int kStepThreads = 256;
 
 // Threads are RG row groups x CL column units of V columns; a unit walks the key channels rg, rg + RG, ...  The first kAhead state
-// rows of a unit are requested before the gates are formed: one decoded token is a chain of latencies (64 sequences x 8 heads x
-// 64 x 64: 8.4 us, 10.5 with the rows behind the gates; 128 x 16 x 128 x 128: 55 and 78).
-// With eight of them in registers fewer CTAs fit an SM, so units with fewer rows have a form with one or four (256 x 16 x 32 x 32:
-// 28 us, in the form with eight 38).
+// rows of a unit are requested before the gates are formed: one decoded token is a chain of latencies.  The rows cost registers, so
+// units with fewer have a form with one or four, and three CTAs fit an SM (six with one row).  256 sequences x 16 heads x 128 x 128: 87 us, with
+// the rows behind the gates 151, with eight ahead and two CTAs an SM 100; 64 x 8 x 64 x 64: 5.1, 8.6 and 7.2; 256 x 16 x 32 x 32: 17, 28 and 38.
 template <typename T, int V, int kAhead>
 __global__ void __launch_bounds__(kStepThreads, V == 4 && kAhead == 1 ? 6 : 3) recurrence_step_kernel(const RecArgs a, int CL) {
   extern __shared__ float sm[];

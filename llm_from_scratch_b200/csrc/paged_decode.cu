@@ -528,7 +528,7 @@ paged_decode_bf16_kernel(const DecodeArgs a) {
 // column per thread of one sequence; most sequences are not cut and leave at once.  Bound by the chain of its loads: who was cut,
 // maxima and sums of all pieces at once into shared memory, and meanwhile the first four pieces of the column.  Sums run over
 // the pieces in their order.  (Piece after piece, with four columns per thread, the latent decode of
-// 8 x 2,000 tokens took 49 us as a whole, this form 25; 128 x 64 .. 1,024 tokens at 16/4 heads x 64 20.7 and 18.9.)
+// 8 x 2,000 tokens took 50 us as a whole, this form 22; 128 x 64 .. 1,024 tokens at 16/4 heads x 64 17.1 and 15.7.)
 constexpr int kCombineThreads = 256;
 constexpr int kCombineAhead = 4;     // pieces of a column in flight
 // pieces whose maxima, sums and weights are held in shared memory at a time
