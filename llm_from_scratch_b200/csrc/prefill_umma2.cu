@@ -91,12 +91,6 @@ struct Args2 {
   bool beside_store;     // the launch before this one is the scatter of its keys and values
 };
 
-// Started beside the launch before it (the step's scatter of keys and values, which nothing here reads): a CTA does not end
-// before that has ended, so that what follows in the stream finds its rows.  Returns at once in an ordinary launch.
-__device__ __forceinline__ void end_behind_store(int tid) {
-  if (tid == 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
-}
-
 template <int DQK, int DV, bool TAIL, bool WINDOW, bool SIGM>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_umma2_kernel(const Args2 a, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,

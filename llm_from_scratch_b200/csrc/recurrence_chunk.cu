@@ -434,9 +434,15 @@ __global__ void __launch_bounds__(4 * D, D == 64 ? 2 : 1) recurrence_chunk_kerne
 template <int D>
 int launch(const RecArgs& a, const ScanArgs& sc, int64_t segments, bool chained, cudaStream_t s) {
   constexpr int smem = sizeof(ChunkSmem<D>);
-  if (cudaFuncSetAttribute(recurrence_chunk_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-      cudaFuncSetAttribute(recurrence_chunk_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-    return B200_ERR_LAUNCH;
+  static bool configured[64] = {false};       // racing threads set the same attributes
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !configured[dev]) {
+    if (cudaFuncSetAttribute(recurrence_chunk_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaFuncSetAttribute(recurrence_chunk_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+      return B200_ERR_LAUNCH;
+    if (dev >= 0 && dev < 64) configured[dev] = true;
+  }
   // segments of uncut sequences are the sequences: no CTA without work in the middle of the grid
   const dim3 grid(static_cast<unsigned>(chained ? segments : sc.n), a.H);
   if (chained) {

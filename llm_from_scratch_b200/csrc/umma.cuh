@@ -242,4 +242,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, volati
 }
 
 }  // namespace umma
+
+// A prompt's attention started beside the launch before it (the step's scatter of keys and values, which it does not read): a CTA does
+// not end before that has ended, so that what follows in the stream finds its rows.  Returns at once in an ordinary launch.
+__device__ __forceinline__ void end_behind_store(int tid) {
+  if (tid == 0) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
 }  // namespace b200
