@@ -525,12 +525,16 @@ paged_decode_bf16_kernel(const DecodeArgs a) {
 }
 
 // Merges the partial results of sequences that were cut across CTAs; zero-fills rows whose context is empty.  A CTA takes one float4
-// column per thread of one sequence; most sequences are not cut and leave at once.  Bound by the chain of its loads: who was cut,
+// column per thread of one sequence (and further ones in large batches); most sequences are not cut and leave at once.  Bound by the chain of its loads: who was cut,
 // maxima and sums of all pieces at once into shared memory, and meanwhile the first four pieces of the column.  Sums run over
 // the pieces in their order.  (Piece after piece, with four columns per thread, the latent decode of
 // 8 x 2,000 tokens took 50 us as a whole, this form 22; 128 x 64 .. 1,024 tokens at 16/4 heads x 64 17.1 and 15.7.)
 constexpr int kCombineThreads = 256;
 constexpr int kCombineAhead = 4;     // pieces of a column in flight
+// CTAs of the launch at most: large batches are hardly cut, and CTAs that only find that out are the launch (512 latent contexts of 16 tokens, 32
+// heads: 41.2 us with a CTA per 1,024 columns, 38.3 so); with fewer, one long context among many waits for its columns (240 of 64 and one of 8,000, 32
+// heads: 1.09 times with this line, 1.30 with half of it).
+constexpr int kCombineCtas = 2368;
 // pieces whose maxima, sums and weights are held in shared memory at a time
 inline int combine_parts(int Hq) { return Hq >= 256 ? 8 : Hq >= 64 ? 16 : 32; }
 
@@ -543,14 +547,13 @@ paged_decode_combine_kernel(const DecodeArgs a, int P) {
   // launched early (programmatic dependent of the attention kernel): everything below reads its results
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const int i = blockIdx.x, n = a.Hq * a.D, tid = threadIdx.x;
-  const int col = (blockIdx.y * kCombineThreads + tid) * 4;            // D is a multiple of 16 on this path
-  const bool in = col < n;
-  __nv_bfloat16* op = static_cast<__nv_bfloat16*>(a.out) + static_cast<int64_t>(i) * n + col;
+  const int step = gridDim.y * kCombineThreads * 4;
+  int col = (blockIdx.y * kCombineThreads + tid) * 4;                  // D is a multiple of 16 on this path
+  __nv_bfloat16* row = static_cast<__nv_bfloat16*>(a.out) + static_cast<int64_t>(i) * n;
   const int64_t len = a.lens[i];
   const int first = a.seq_info[2 * i], last = a.seq_info[2 * i + 1];
   if (len <= 0) {
-    if (in)
-      for (int e = 0; e < 4; ++e) op[e] = __float2bfloat16_rn(0.f);
+    for (; col < n; col += step) *reinterpret_cast<uint2*>(row + col) = make_uint2(0u, 0u);
     return;
   }
   if (first < 0) return;
@@ -560,7 +563,7 @@ paged_decode_combine_kernel(const DecodeArgs a, int P) {
   auto load = [&](int p0) {
 #pragma unroll
     for (int u = 0; u < kCombineAhead; ++u)
-      if (in && p0 + u < np) x[u] = __ldcg(reinterpret_cast<const float4*>(a.part_o + slot_of(p0 + u) * n + col));
+      if (col < n && p0 + u < np) x[u] = __ldcg(reinterpret_cast<const float4*>(a.part_o + slot_of(p0 + u) * n + col));
   };
   load(0);
   auto stage = [&](int p0) {         // maxima and sums of the pieces p0 ..; a context of more than P pieces passes three times
@@ -594,28 +597,32 @@ paged_decode_combine_kernel(const DecodeArgs a, int P) {
       s_inv[h] = L;
     }
   }
-  const int head = in ? col / a.D : 0;
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int p0 = 0; p0 < np; p0 += P) {
-    if (!once) stage(p0);
-    else __syncthreads();
-    const int pc = min(P, np - p0);
-    for (int t = tid; t < pc * a.Hq; t += kCombineThreads) s_w[t] = exp2f(s_ml[t].x - s_M[t % a.Hq]) * s_inv[t % a.Hq];
-    __syncthreads();
-    for (int q0 = 0; q0 < pc; q0 += kCombineAhead) {
+  for (int c0 = col - tid * 4; c0 < n; c0 += step, col += step) {      // the same trips for every thread
+    const bool in = col < n;
+    const int head = in ? col / a.D : 0;
+    if (c0 >= step) load(0);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int p0 = 0; p0 < np; p0 += P) {
+      if (!once) stage(p0);
+      else __syncthreads();
+      const int pc = min(P, np - p0);
+      for (int t = tid; t < pc * a.Hq; t += kCombineThreads) s_w[t] = exp2f(s_ml[t].x - s_M[t % a.Hq]) * s_inv[t % a.Hq];
+      __syncthreads();
+      for (int q0 = 0; q0 < pc; q0 += kCombineAhead) {
 #pragma unroll
-      for (int u = 0; u < kCombineAhead; ++u)
-        if (in && q0 + u < pc) {
-          const float w = s_w[(q0 + u) * a.Hq + head];
-          acc.x += w * x[u].x;
-          acc.y += w * x[u].y;
-          acc.z += w * x[u].z;
-          acc.w += w * x[u].w;
-        }
-      load(p0 + q0 + kCombineAhead);
+        for (int u = 0; u < kCombineAhead; ++u)
+          if (in && q0 + u < pc) {
+            const float w = s_w[(q0 + u) * a.Hq + head];
+            acc.x += w * x[u].x;
+            acc.y += w * x[u].y;
+            acc.z += w * x[u].z;
+            acc.w += w * x[u].w;
+          }
+        load(p0 + q0 + kCombineAhead);
+      }
     }
+    if (in) *reinterpret_cast<uint2*>(row + col) = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
   }
-  if (in) *reinterpret_cast<uint2*>(op) = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
 }
 
 // The combine follows the attention kernel in the stream and reads only what that kernel wrote: as a
@@ -623,7 +630,8 @@ paged_decode_combine_kernel(const DecodeArgs a, int P) {
 int launch_combine(const DecodeArgs& a, int batch, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   const int P = combine_parts(a.Hq);
-  cfg.gridDim = dim3(batch, (a.Hq * a.D / 4 + kCombineThreads - 1) / kCombineThreads);
+  const int cols = (a.Hq * a.D / 4 + kCombineThreads - 1) / kCombineThreads;
+  cfg.gridDim = dim3(batch, batch >= kCombineCtas ? 1 : cols < kCombineCtas / batch ? cols : kCombineCtas / batch);
   cfg.blockDim = dim3(kCombineThreads);
   cfg.dynamicSmemBytes = (3 * P + 2) * a.Hq * sizeof(float);
   cfg.stream = s;

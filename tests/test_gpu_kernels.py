@@ -211,6 +211,36 @@ def test_a_broken_key_row_is_seen_in_the_output(dtype, D, page, n, at):
     assert torch.isfinite(got[0, :4]).all() and torch.isnan(got[0, 4:]).all()
 
 
+@pytest.mark.parametrize("latent", [False, True])
+def test_merge_of_one_long_context_in_a_large_batch(latent):
+    """The merge's CTAs take several columns each where there are many, and the long context has more pieces than fit their shared
+    memory at a time; empty contexts are zeros."""
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    lens = [64] * (240 if latent else 1024)
+    lens[7], lens[3], lens[-1] = 9000, 0, 33
+    case = deal_blocks(lens, 16, np.random.default_rng(3), pad_blocks=1)
+    tables, ctx = torch.from_numpy(case.block_tables).cuda(), torch.from_numpy(case.context_lens).cuda()
+    if latent:
+        H, cache, qa, qr = 32, r(case.num_blocks, 16, 576), r(len(lens), 32, 512), r(len(lens), 32, 64)
+        got = ops.mla_decode(qa, qr, cache, tables, ctx, 0.07)
+    else:
+        H, q, kc, vc = 64, r(len(lens), 64, 64), r(case.num_blocks, 16, 8, 64), r(case.num_blocks, 16, 8, 64)
+        got = ops.paged_decode_gqa(q, kc, vc, tables, ctx, 0.125)
+    ops.check_status()
+    assert (got[3] == 0).all()
+    for i in (0, 6, 7, 8, len(lens) - 1):
+        rows = (tables[i, :-(-lens[i] // 16)].long()[:, None] * 16 + torch.arange(16, device="cuda")).flatten()[:lens[i]]
+        if latent:
+            keys = cache.view(-1, 576)[rows].double()
+            want = torch.softmax((qa[i].double() @ keys[:, :512].T + qr[i].double() @ keys[:, 512:].T) * 0.07, -1) @ keys[:, :512]
+        else:
+            k, v = (c.view(-1, 8, 64)[rows].double().repeat_interleave(8, 1) for c in (kc, vc))
+            want = torch.einsum("hn,nhd->hd", torch.softmax(torch.einsum("hd,nhd->hn", q[i].double(), k) * 0.125, -1), v)
+        assert_close(got[i], want, torch.bfloat16)
+
+
 def test_paged_decode_bf16_single_short_sequence_and_stale_table_entries():
     # entries past ceil(len/16) hold stale ids outside the pool: they must never be read
     case, q, kc, vc = _decode_case([20], 32, 8, 128, 16, torch.bfloat16, seed=3)
