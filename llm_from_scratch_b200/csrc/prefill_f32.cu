@@ -307,7 +307,7 @@ int launch_rows(const PrefillF32Args& a, int max_seqlen_q, int64_t total_q, cuda
 // 16/16 x 128: 172 and 302; 256 x 1 behind 64 at 16/4 x 64: 100 and 61.
 bool general_is_faster(const PrefillF32Args& a, int D, int64_t total_q, int max_seqlen_q, int max_seqlen_k) {
   const int64_t rows = static_cast<int64_t>(max_seqlen_q) * (a.Hq / a.Hkv);
-  if (rows > 32 || max_seqlen_k > 128) return false;
+  if (rows > 32 || max_seqlen_k > 128 || a.num_seqs > 65535 || a.Hq > 65535) return false;      // the latter two: its grid
   const double rate = max_seqlen_q == 1 ? 1600 : max_seqlen_q <= 3 ? 2100 : 3100;                   // rows x keys a us
   const double all = static_cast<double>(total_q) * a.Hq * (max_seqlen_k - max_seqlen_q / 2) / rate;
   const double chain = 0.75 * max_seqlen_k, general = 2.5 + (all > chain ? all : chain);

@@ -80,6 +80,14 @@ def test_short_portions(Hq, Hkv, D, n, q_len, prefix):
     ops.check_status()
 
 
+def test_more_sequences_than_a_grid_of_the_general_kernel_holds():
+    from llm_from_scratch_b200 import ops
+    n = 70000
+    q, k, v, cu = _randn(1, n, 2, 32), _randn(2, n, 1, 32), _randn(3, n, 1, 32), torch.arange(n + 1, dtype=torch.int32, device="cuda")
+    assert torch.equal(ops.prefill_varlen(q, k, v, cu, cu, 1, 1, 0.2), v.expand(n, 2, 32))
+    ops.check_status()
+
+
 def test_values_a_row_does_not_see_stay_out_of_it():
     from llm_from_scratch_b200 import ops
     lens, Hq, Hkv, D = [100, 90], 8, 2, 64
